@@ -54,8 +54,4 @@ inline bool fuse_r2c_enabled()
                 return launch_codelet_t<S_, false, true>(a, st);                        \
         return launch_codelet_t<S_>(a, st);                                              \
     }                                                                                    \
-    int launch_coltile_##ID(const ColArgs* a, cudaStream_t st)                           \
-    {                                                                                    \
-        return launch_coltile_t<CodeletSpec<ID>::type>(a, st);                           \
-    }                                                                                    \
     }

@@ -83,6 +83,7 @@ using namespace gfft;
 extern "C" int gfft_launch_row(const RowArgs* a, void* stream)
 {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (a->tile) return gfft_launch_tile_row(a, stream);
     switch (a->codelet) {
     case -1: break;
 #define GFFT_CASE_ROW(ID, ...) \
@@ -101,14 +102,7 @@ extern "C" int gfft_launch_row(const RowArgs* a, void* stream)
 extern "C" int gfft_launch_col(const ColArgs* a, void* stream)
 {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    switch (a->codelet) {
-    case -1: break;
-#define GFFT_CASE_COL(ID, ...) \
-    case ID: return launch_coltile_##ID(a, st);
-        GFFT_CODELETS(GFFT_CASE_COL)
-#undef GFFT_CASE_COL
-    default: return (int)cudaErrorInvalidValue;
-    }
+    if (a->tile) return gfft_launch_tile_col(a, stream);
     switch (a->ip.rmax) {
     case 16: return launch_col_r16(a, st);
     case 47: return launch_col_r47(a, st);

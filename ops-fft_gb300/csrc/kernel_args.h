@@ -88,6 +88,10 @@ struct RowArgs {
     // (pinned host buffers): slots are filled by per-thread cp.async instead
     // of bulk copies
     int32_t host_in;
+    // register-to-register rows of any length with radices <= 16
+    // (csrc/tile_fft.cuh): tfpc rows per CTA, one exchange buffer of
+    // tfpc * lpad float2 or two (nbuf); twiddles are read from global memory
+    int32_t tile;
 };
 
 // Strided ("column") transforms, optionally one outer Stockham pass of a
@@ -120,14 +124,16 @@ struct ColArgs {
     int32_t conj_out;
     int32_t staged_out;  // output of column c is out + c*L + k (contiguous blocks)
     float scale;
-    // column-tile codelet (codelet >= 0): tfpc adjacent columns per tile, one
-    // codelet transform group per column, column g held at g*wsize in shared
-    // memory after the pass-table window [tw_lo, tw_lo + tw_cnt)
-    int32_t codelet;
-    int32_t tw_lo;
-    int32_t tw_cnt;
-    int32_t wsize;
     int32_t smem_bytes;
+    // register-to-register tiles of any length with radices <= 16
+    // (csrc/tile_fft.cuh): tfpc columns per CTA, exchange buffers (nbuf) of
+    // wsize float2, padded by one element every 2^pshift; with otw2d the
+    // outer twiddles come from one table (entry r*ons + j) at otw_hi
+    int32_t tile;
+    int32_t wsize;
+    int32_t pshift;
+    int32_t spitch;  // staged_out: shared pitch of one column
+    int32_t otw2d;
     int32_t pad2_;
 };
 
@@ -355,6 +361,8 @@ int gfft_launch_dpass(const gfft::DPassArgs* a, void* stream);
 int gfft_gen_dtwiddles(void* table, long long n, void* stream);
 int gfft_launch_row(const gfft::RowArgs* a, void* stream);
 int gfft_launch_col(const gfft::ColArgs* a, void* stream);
+int gfft_launch_tile_row(const gfft::RowArgs* a, void* stream);
+int gfft_launch_tile_col(const gfft::ColArgs* a, void* stream);
 int gfft_launch_pack(const gfft::PackArgs* a, void* stream);
 int gfft_launch_tc(const gfft::TcArgs* a, void* stream);
 int gfft_launch_ragged(const gfft::RagArgs* a, void* stream);

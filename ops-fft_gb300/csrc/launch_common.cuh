@@ -106,35 +106,8 @@ int launch_codelet_t(const RowArgs* a, cudaStream_t st)
     return (int)launch_pdl(codelet_kernel<S, FC2R, FR2C>, dim3((unsigned)grid), dim3(threads), (size_t)a->smem_bytes, st, *a);
 }
 
-template <class S>
-int launch_coltile_t(const ColArgs* a, cudaStream_t st)
-{
-    static unsigned long long attr_mask = 0;
-    static thread_local int last_threads = -1, last_smem = -1, last_occ = 1;
-    const int threads = S::NTHR * a->tfpc;
-    if (a->ip.L != S::L || a->tfpc < 1 || threads > S::MAXT || a->ncols <= 0 || a->wsize <= 0)
-        return (int)cudaErrorInvalidValue;
-    if (a->smem_bytes <= 0 || a->smem_bytes > kMaxSmemBytes) return (int)cudaErrorInvalidValue;
-    cudaError_t e = ensure_smem_attr(coltile_kernel<S>, attr_mask, (size_t)a->smem_bytes);
-    if (e != cudaSuccess) return (int)e;
-    if (threads != last_threads || a->smem_bytes != last_smem) {
-        int occ = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, coltile_kernel<S>, threads, (size_t)a->smem_bytes);
-        if (e != cudaSuccess) return (int)e;
-        last_threads = threads;
-        last_smem = a->smem_bytes;
-        last_occ = occ < 1 ? 1 : occ;
-    }
-    const int64_t ntiles = (a->ncols + a->tfpc - 1) / a->tfpc;
-    int64_t grid = (int64_t)sm_count() * last_occ;
-    if (grid < 1) grid = 1;
-    if (grid > ntiles) grid = ntiles;
-    return (int)launch_pdl(coltile_kernel<S>, dim3((unsigned)grid), dim3(threads), (size_t)a->smem_bytes, st, *a);
-}
-
-#define GFFT_DECL_LAUNCH(ID, ...)                           \
-    int launch_codelet_##ID(const RowArgs* a, cudaStream_t st); \
-    int launch_coltile_##ID(const ColArgs* a, cudaStream_t st);
+#define GFFT_DECL_LAUNCH(ID, ...) \
+    int launch_codelet_##ID(const RowArgs* a, cudaStream_t st);
 GFFT_CODELETS(GFFT_DECL_LAUNCH)
 #undef GFFT_DECL_LAUNCH
 int launch_row_r16(const RowArgs* a, cudaStream_t st);

@@ -1,0 +1,121 @@
+// tile_fft.cu - launchers of the tile kernel (instances in tile_io*.cu).
+#include "launch_common.cuh"
+#include "tile_fft.cuh"
+
+namespace gfft {
+int launch_tile_io0(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+int launch_tile_io0w(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+int launch_tile_io1(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+int launch_tile_io2(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+int launch_tile_io3(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+int launch_tile_io4(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+
+namespace {
+
+int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
+{
+    int threads = t.W * t.ip.nthr;
+    threads = (threads + 31) & ~31;
+    if (t.W < 1 || t.ip.nthr < 1 || threads > kTileMaxThreads || t.ncols == 0 || smem > (size_t)kMaxSmemBytes)
+        return (int)cudaErrorInvalidValue;
+    const unsigned grid = (t.ncols + (unsigned)t.W - 1) / (unsigned)t.W;
+    switch (io) {
+    case IO_C2C:
+        // the span of one transform decides the offset width
+        if ((int64_t)t.ip.L * (t.in_st8 > t.out_st8 ? t.in_st8 : t.out_st8) > 0xffffffffll)
+            return launch_tile_io0w(t, threads, smem, grid, st);
+        return launch_tile_io0(t, threads, smem, grid, st);
+    case IO_R2C_EVEN: return launch_tile_io1(t, threads, smem, grid, st);
+    case IO_C2R_EVEN: return launch_tile_io2(t, threads, smem, grid, st);
+    case IO_R2C_ODD: return launch_tile_io3(t, threads, smem, grid, st);
+    case IO_C2R_ODD: return launch_tile_io4(t, threads, smem, grid, st);
+    default: return (int)cudaErrorInvalidValue;
+    }
+}
+
+constexpr int64_t kTileMaxCols = (int64_t(1) << 31) - 64;  // 32-bit column arithmetic
+
+}  // namespace
+}  // namespace gfft
+
+using namespace gfft;
+
+extern "C" int gfft_launch_tile_row(const RowArgs* a, void* stream)
+{
+    if (a->ntf < 1 || a->ntf > kTileMaxCols) return (int)cudaErrorInvalidValue;
+    TileArgs t{};
+    t.ip = a->ip;
+    t.tw = static_cast<const float2*>(a->tw);
+    t.post = static_cast<const float2*>(a->post_tw);
+    t.in = a->in;
+    t.out = a->out;
+    t.ncols = (uint32_t)a->ntf;
+    t.cpi = t.in_split = t.out_split = t.tw_div = t.ons = tile_div(1);
+    t.T = tile_div(a->ip.nthr);
+    t.in_dist = a->in_dist;
+    t.out_dist = a->out_dist;
+    t.in_st8 = t.out_st8 = 8;
+    t.W = a->tfpc;
+    t.rows = 1;
+    t.emul = 1;
+    t.cmul = a->lpad;
+    t.pshift = a->pshift;
+    t.nbuf = a->nbuf;
+    t.bufsz = a->tfpc * a->lpad;
+    t.conj_in = a->conj_in;
+    t.conj_out = a->conj_out;
+    t.weight = a->weight;
+    t.nreal = a->nreal;
+    t.scale = a->scale;
+    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int gfft_launch_tile_col(const ColArgs* a, void* stream)
+{
+    if (a->ncols < 1 || a->ncols > kTileMaxCols) return (int)cudaErrorInvalidValue;
+    TileArgs t{};
+    t.ip = a->ip;
+    t.tw = static_cast<const float2*>(a->tw);
+    if (a->ons > 1) {
+        if (a->otw2d) {
+            t.otw = static_cast<const float2*>(a->otw_hi);
+        } else {
+            t.otw_hi = static_cast<const float2*>(a->otw_hi);
+            t.otw_lo = static_cast<const float2*>(a->otw_lo);
+        }
+    }
+    t.otw_shift = a->otw_shift;
+    t.in = a->in;
+    t.out = a->out;
+    t.ncols = (uint32_t)a->ncols;
+    // a split at or beyond the columns of an item never divides
+    t.cpi = tile_div(a->cpi);
+    t.in_split = tile_div(a->in_split < a->cpi ? a->in_split : a->cpi);
+    t.out_split = tile_div(a->out_split < a->cpi ? a->out_split : a->cpi);
+    t.tw_div = tile_div(a->tw_div < a->cpi ? a->tw_div : a->cpi);
+    t.ons = tile_div(a->ons);
+    t.T = tile_div(a->ip.nthr);
+    t.in_dist = a->in_dist;
+    t.in_hi = a->in_hi;
+    t.in_lo = a->in_lo;
+    t.in_st8 = 8 * a->in_stride;
+    t.out_dist = a->out_dist;
+    t.out_hi = a->out_hi;
+    t.out_lo = a->out_lo;
+    t.out_st8 = 8 * a->out_stride;
+    t.W = a->tfpc;
+    while ((1 << t.wshift) < t.W) ++t.wshift;
+    if ((1 << t.wshift) != t.W) return (int)cudaErrorInvalidValue;
+    t.rows = 0;
+    t.emul = a->tfpc;
+    t.cmul = 1;
+    t.pshift = a->pshift;
+    t.nbuf = a->nbuf;
+    t.bufsz = a->wsize;
+    t.staged_out = a->staged_out;
+    t.spitch = a->spitch;
+    t.conj_in = a->conj_in;
+    t.conj_out = a->conj_out;
+    t.scale = a->scale;
+    return launch_tile(IO_C2C, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
+}

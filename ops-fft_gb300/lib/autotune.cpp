@@ -112,7 +112,7 @@ std::string signature(const StepList& sl)
             for (int p = 0; p < s.row.ip.npass; ++p) os << s.row.ip.pass[p].radix << '.';
             break;
         case Step::COL:
-            os << s.col.codelet << ',' << s.col.tfpc << ',';
+            os << s.col.tile << ',' << s.col.tfpc << ',';
             for (int p = 0; p < s.col.ip.npass; ++p) os << s.col.ip.pass[p].radix << '.';
             break;
         case Step::CLUSTER: os << s.cl.kid << ',' << s.cl.csize; break;

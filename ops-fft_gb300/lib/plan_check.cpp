@@ -67,12 +67,49 @@ int buffers_used(int npass, int start, bool last_global)
     return used;
 }
 
+// Tile kernel (csrc/tile_fft.cuh): every shared index of every pass, as the
+// kernel computes it, inside the exchange buffer and injective per pass.
+bool check_tile(const InnerPlan& ip, int W, int emul, int cmul, int ps, int64_t bufsz, int nbuf, int64_t smem_bytes,
+                bool first_reads, std::string& why)
+{
+    if (ip.rmax != 16 || W < 1 || W * ip.nthr > 512) return fail(why, "tile threads");
+    if (nbuf != 1 && nbuf != 2) return fail(why, "tile buffers");
+    if (nbuf * bufsz * 8 > smem_bytes || smem_bytes > kMaxSmemBytes) return fail(why, "tile smem");
+    auto pad = [&](int i) { return i + (i >> ps); };
+    const int L = ip.L;
+    if (W > 1 && emul == 1 && cmul < pad(L - 1) + 1) return fail(why, "tile pitch");
+    if (emul > 1 && (emul != W || cmul != 1)) return fail(why, "tile columns");
+    for (int p = 0; p < ip.npass; ++p) {
+        const PassDesc& d = ip.pass[p];
+        const int R = d.radix, nbf = L / R, ns = d.ns;
+        const int nb = R >= 16 ? 1 : 16 / R;
+        if ((int64_t)nb * ip.nthr < nbf) return fail(why, "tile threads do not cover a pass");
+        for (int j = 0; j < nbf; ++j) {
+            for (int r = 0; r < R; ++r) {
+                if ((p > 0 || first_reads) && pad(j) + r * (nbf + (nbf >> ps)) != pad(j + r * nbf)) return fail(why, "tile read stride");
+                if (p + 1 < ip.npass) {
+                    const int i0 = j / ns * ns * R + j % ns, ws = ns == 1 ? 1 : ns + (ns >> ps);
+                    if (pad(i0) + r * ws != pad(i0 + r * ns)) return fail(why, "tile write stride");
+                }
+            }
+        }
+    }
+    if ((int64_t)pad(L - 1) * emul + (int64_t)(W - 1) * cmul >= bufsz) return fail(why, "tile exchange buffer");
+    return true;
+}
+
 bool check_row(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
 {
     const RowArgs& a = s.row;
     if (!check_inner(a.ip, tw_count, why)) return false;
     const int L = a.ip.L;
     const int maxthr = a.ip.rmax == 16 ? 512 : 256;
+    if (a.tile) {
+        if (a.codelet >= 0 || a.staged || a.host_in) return fail(why, "tile row mode");
+        if (a.ntf >= (int64_t(1) << 31) - 64) return fail(why, "tile rows");
+        if (!check_tile(a.ip, a.tfpc, 1, a.lpad, a.pshift, (int64_t)a.tfpc * a.lpad, a.nbuf, a.smem_bytes,
+                        a.io_mode == IO_C2R_EVEN, why)) return false;
+    } else {
     if (a.codelet < 0 && (a.ip.nthr * a.tfpc > maxthr || a.tfpc < 1)) return fail(why, "row threads");
     if (a.tfpc < 1) return fail(why, "row tile");
     if (a.nstage < 1 || a.nstage > 4) return fail(why, "row stages");
@@ -90,8 +127,10 @@ bool check_row(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
         const int ps = (cr[0] % 2 == 0) ? 4 : 30;
         if (a.pshift != ps) return fail(why, "codelet padding");
     }
+    }
     const bool even = a.io_mode == IO_R2C_EVEN || a.io_mode == IO_C2R_EVEN;
     const int maxidx = even ? L : L - 1;
+    if (!a.tile) {
     if (maxidx + (maxidx >> a.pshift) >= a.lpad) return fail(why, "row lpad too small");
     const int64_t row_bytes = a.in_dist * a.in_esize;
     if ((int64_t)a.tfpc * row_bytes > a.stage_bytes || a.stage_bytes % 16) return fail(why, "row stage too small");
@@ -133,6 +172,7 @@ bool check_row(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
         if (buffers_used(a.ip.npass, start, last_global) > a.nbuf) return fail(why, "row needs more shared buffers");
     }
     if (a.staged && (int64_t)a.tfpc * (L + 1) >= (1 << 22)) return fail(why, "staged copy index range");
+    }
     int64_t in_last = 0, out_last = 0, in_es = 8, out_es = 8;
     const int N = a.nreal;
     switch (a.io_mode) {
@@ -162,28 +202,11 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
     const ColArgs& a = s.col;
     if (!check_inner(a.ip, tw_count, why)) return false;
     const int L = a.ip.L;
-    if (a.codelet >= 0) {
-        // column-tile codelet: the codelet's compile-time spec must match the plan
-        int cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
-        if (gfft_codelet_info(a.codelet, &cl, &cn, cr, &cnr, &cmaxt, &cminb) != 0 || cl != L)
-            return fail(why, "coltile codelet id");
-        if (cn != a.ip.nthr || cnr != a.ip.npass) return fail(why, "coltile spec");
-        for (int q = 0; q < cnr; ++q)
-            if (cr[q] != a.ip.pass[q].radix) return fail(why, "coltile radices");
-        if (a.tfpc < 1 || a.tfpc * cn > cmaxt) return fail(why, "coltile threads");
-        const int pshift = (cr[0] % 2 == 0) ? 4 : 30;
-        const int64_t need = (int64_t)(L - 1) + ((int64_t)(L - 1) >> pshift) + 1;
-        if (a.wsize < need) return fail(why, "coltile column region");
-        const int64_t tw_bytes = ((int64_t)a.tw_cnt * 8 + 127) & ~(int64_t)127;
-        if (tw_bytes + (int64_t)a.tfpc * a.wsize * 8 > a.smem_bytes || a.smem_bytes > kMaxSmemBytes)
-            return fail(why, "coltile smem");
-        if (a.tw_cnt < 0 || a.tw_lo < 0 || a.tw_lo + (int64_t)a.tw_cnt > tw_count) return fail(why, "coltile tw window");
-        for (int q = 0; q < a.ip.npass; ++q)
-            if (a.ip.pass[q].ns > 1 && a.tw_cnt > 0 &&
-                (a.ip.pass[q].tw_off < a.tw_lo ||
-                 a.ip.pass[q].tw_off + (int64_t)a.ip.pass[q].ns * a.ip.pass[q].radix > (int64_t)a.tw_lo + a.tw_cnt))
-                return fail(why, "coltile tw window misses a pass table");
-        if (a.ons > 1 || a.staged_out) return fail(why, "coltile with outer twiddles or staged output");
+    if (a.tile) {
+        if (a.tfpc & (a.tfpc - 1)) return fail(why, "tile column mode");
+        if (a.ncols >= (int64_t(1) << 31) - 64) return fail(why, "tile columns");
+        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, false, why)) return false;
+        if (a.staged_out && (a.spitch < L || (int64_t)a.tfpc * a.spitch > a.wsize)) return fail(why, "tile staging");
     } else {
         const int maxthr = a.ip.rmax == 16 ? 512 : 256;
         if (a.ip.nthr * a.tfpc > maxthr || a.tfpc < 1 || a.tfp < a.tfpc) return fail(why, "col threads");
@@ -207,6 +230,11 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
     if (a.ons > 1) {
         const int64_t M = a.ons * L;
         if (M >= (int64_t(1) << 32)) return fail(why, "outer twiddle index overflow");
+        if (a.tw_div < 1) return fail(why, "tw_div");
+        if (a.otw2d) {
+            if (!a.tile || s.hi_off < 0 || s.hi_off + M > tw_count) return fail(why, "outer twiddle table");
+            return true;
+        }
         const int64_t S = int64_t(1) << a.otw_shift;
         if (s.lo_off < 0 || s.lo_off + S > tw_count) return fail(why, "outer lo table");
         if (s.hi_off < 0 || s.hi_off + (M + S - 1) / S > tw_count) return fail(why, "outer hi table");

@@ -189,6 +189,10 @@ int row_nbuf(int npass, int start, bool last_global)
 // Hints of the problem being planned (set by build_steps for its duration).
 thread_local const PlanHints* t_hints = nullptr;
 
+// Plans without tiles (set for its duration): the allocation-free path, whose
+// twiddles live in a fixed array.
+thread_local bool t_no_tiles = false;
+
 struct HintScope {
     explicit HintScope(const PlanHints* h) : prev(t_hints) { t_hints = h; }
     ~HintScope() { t_hints = prev; }
@@ -220,6 +224,74 @@ bool clusters_enabled()
 }
 
 namespace {
+
+// ------------------------------------------------------------ tile kernel
+// (csrc/tile_fft.cuh)
+constexpr int kTileMaxThreads = 512;
+constexpr int kTileElems = 16;  // elements a thread holds
+constexpr int64_t kTileMaxCols = (int64_t(1) << 31) - 64;  // 32-bit column arithmetic
+
+int tile_threads(int L, const std::vector<int>& rad)
+{
+    int t = 1;
+    for (int r : rad) {
+        const int nb = r >= kTileElems ? 1 : kTileElems / r;
+        t = std::max(t, (int)ceil_div(L / r, nb));
+    }
+    return t;
+}
+
+// Radices for the tile kernel: fewest passes, then fewest threads, then
+// balanced; an odd radix (or a power of two) first, which keeps the shared
+// addresses of a butterfly an arithmetic sequence, the others descending.
+// c2r: the first pass reads the exchange buffer too (the Hermitian
+// pre-process wrote it), so L/R0 has to be a multiple of a power-of-two R0.
+std::vector<int> choose_tile_radices(int L, bool c2r = false)
+{
+    if (L == 1) return {1};
+    std::vector<int> best, cur;
+    int best_np = 1 << 30, best_t = 0, best_min = 0;
+    std::function<void(int, int)> dfs = [&](int rem, int maxr) {
+        if ((int)cur.size() > best_np || (int)cur.size() >= kMaxPass) return;
+        if (rem == 1) {
+            const int np = (int)cur.size(), t = tile_threads(L, cur);
+            const int mn = *std::min_element(cur.begin(), cur.end());
+            if (np < best_np || (np == best_np && (t < best_t || (t == best_t && mn > best_min)))) {
+                best = cur;
+                best_np = np;
+                best_t = t;
+                best_min = mn;
+            }
+            return;
+        }
+        for (int r = std::min(maxr, kTileElems); r >= 2; --r) {
+            if (rem % r) continue;
+            cur.push_back(r);
+            dfs(rem / r, r);
+            cur.pop_back();
+        }
+    };
+    dfs(L, kTileElems);
+    if (best.size() > 1) {
+        auto pow2 = [&](int r) { return (r & (r - 1)) == 0 && (!c2r || (L / r) % r == 0); };
+        size_t first = best.size();
+        for (size_t i = 0; i < best.size() && first == best.size(); ++i)
+            if (best[i] & 1) first = i;
+        for (size_t i = 0; i < best.size() && first == best.size(); ++i)
+            if (pow2(best[i])) first = i;
+        if (first < best.size()) std::rotate(best.begin(), best.begin() + first, best.begin() + first + 1);
+    }
+    return best;
+}
+
+// log2 of the first radix when that is a power of two: the shared padding
+int tile_pshift(int L, const std::vector<int>& rad, bool c2r = false)
+{
+    if (rad.size() < 2 || (rad[0] & (rad[0] - 1)) != 0 || (c2r && (L / rad[0]) % rad[0])) return 30;
+    int s = 0;
+    while ((1 << s) < rad[0]) ++s;
+    return s;
+}
 
 // Score bonus of a codelet configuration with a per-group work buffer
 // (ping-pong passes) over the in-place one.
@@ -369,6 +441,68 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
     return true;
 }
 
+// Rows of any length with radices <= 16 on the tile kernel.
+bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io_mode, int nreal, int weight,
+                        TwiddleBuilder& tb, Step& st)
+{
+    if (ntf >= kTileMaxCols) return false;
+    const std::vector<int> rad = choose_tile_radices(L, io_mode == IO_C2R_EVEN);
+    if (rad.empty()) return false;
+    int T = tile_threads(L, rad);
+    if (T > kTileMaxThreads) return false;
+    // one thread per row reads 8 L bytes of its own: beyond 12 complex
+    // values the row kernel's staged copies are faster (16 x 2^20: 100 against
+    // 129 us; 12 x 1.4M: 84 against 81)
+    if (T == 1 && L > 12 && io_mode == IO_C2C) return false;
+    // few rows: one butterfly a thread and pass (half the instructions on a
+    // row's critical path when its radices are 8 or less) while that leaves
+    // at most 256 threads on an SM
+    int T1 = 1;
+    for (int r : rad) T1 = std::max(T1, L / r);
+    if (T1 <= kTileMaxThreads && ntf * T1 <= 152 * 256) T = T1;
+    TwiddleBuilder trial = tb;
+    st = Step{};
+    st.kind = Step::ROW;
+    RowArgs& a = st.row;
+    if (!build_inner(L, rad, T, trial, a.ip)) return false;
+    const bool even_mode = io_mode == IO_R2C_EVEN || io_mode == IO_C2R_EVEN;
+    if (even_mode) st.post_off = trial.add_linear(L / 2 + 1, 2 * (int64_t)L, 1);
+    const int ps = tile_pshift(L, rad, io_mode == IO_C2R_EVEN);
+    int pitch = L + (L >> ps) + 1;
+    if (T < 16) {
+        while (pitch % 16 != T % 16) ++pitch;
+    } else {
+        pitch += pitch & 1;
+    }
+    // two warps per CTA, more only for longer rows: small CTAs wait for
+    // fewer threads at each barrier (100 x 131072: 36.4 us at 64 threads, 41
+    // at 256; 1024 x 16384: 44.3 against 48.0)
+    const int W = (int)std::max<int64_t>(1, std::min<int64_t>(64 / T, ntf));
+    const int64_t one = (int64_t)W * pitch * 8;
+    if (one > kMaxSmemBytes) return false;
+    tb = trial;
+    a.tile = 1;
+    a.ntf = ntf;
+    a.in_dist = in_dist;
+    a.out_dist = out_dist;
+    a.tfpc = W;
+    a.lpad = pitch;
+    a.nbuf = 1;
+    a.io_mode = io_mode;
+    a.weight = weight;
+    a.nreal = nreal;
+    a.scale = 1.f;
+    a.conj_out = io_mode == IO_C2R_EVEN ? 1 : 0;
+    a.nstage = 1;
+    a.pshift = ps;
+    a.in_esize = io_mode == IO_R2C_ODD ? 4 : 8;
+    a.post_cnt = even_mode ? L / 2 + 1 : 0;
+    a.smem_bytes = (int32_t)one;
+    a.codelet = -1;
+    st.tw_off = 0;
+    return true;
+}
+
 // One on-chip transform per contiguous batch item (persistent row kernel,
 // see csrc/row_pipe.cuh for the shared-memory layout).
 bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io_mode, int nreal, int weight,
@@ -381,6 +515,7 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     int nthr = pick_nthr(L, rad, maxthr);
     int codelet = -1;
     if (make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
+    if (make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
     const bool even_mode = io_mode == IO_R2C_EVEN || io_mode == IO_C2R_EVEN;
     const bool staged = nthr < 32 && (io_mode == IO_C2C || io_mode == IO_R2C_EVEN);
     const int start = io_mode == IO_C2R_EVEN ? 1 : 0;
@@ -480,6 +615,71 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     return a.smem_bytes <= kMaxSmemBytes;
 }
 
+// Turns the column pass described by st.col (addresses filled in) into tiles
+// of the tile kernel; false when it does not apply.
+bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilder& tb, Step& st)
+{
+    ColArgs& a = st.col;
+    if (a.ncols >= kTileMaxCols || t_no_tiles) return false;
+    const std::vector<int> rad = choose_tile_radices(Lq);
+    if (rad.empty()) return false;
+    const int T = tile_threads(Lq, rad);
+    // strided axes: 16 columns (128-byte row segments) where the threads
+    // allow it (512-point axes of 512^3: 1283 us against 1489 at 8 columns;
+    // 256 x 263168: 169 against 313); passes of a long row, whose segments
+    // are neighbours in memory, take 8 and smaller CTAs (131072 x 128: 121
+    // against 127 us).  At least 4: narrower segments waste sectors.
+    int W = S > 1 ? 16 : 8;
+    while (W > 4 && W * T > kTileMaxThreads) W >>= 1;
+    if (T * W > kTileMaxThreads) return false;
+    // few columns: narrower tiles until two CTAs per SM are there
+    while (W > 4 && a.ncols / W < 304) W >>= 1;
+    TwiddleBuilder trial = tb;
+    InnerPlan ip;
+    if (!build_inner(Lq, rad, T, trial, ip)) return false;
+    const int ps = tile_pshift(Lq, rad);
+    const int Lp = Lq + (Lq >> ps);
+    int spitch = 0;
+    int64_t buf = (int64_t)W * Lp;
+    if (staged_out) {
+        spitch = Lq;
+        while (spitch % 16 != 16 / W % 16) ++spitch;
+        buf = std::max<int64_t>(buf, (int64_t)W * spitch);
+    }
+    // one exchange buffer and two barriers a pass: two buffers and one
+    // barrier leave fewer CTAs per SM (512 x 65536 in 64 KB tiles: 161 us
+    // against 116)
+    const int64_t smem = buf * 8;
+    if (smem > kMaxSmemBytes) return false;
+    if (Ns > 1) {
+        const int64_t M = Ns * Lq;
+        // the outer twiddles as one table read like the data (one load an
+        // element, correctly rounded) up to 8 MB, which the L2 holds beside
+        // the data; beyond, the product of two small tables
+        if (M <= (int64_t)1 << 20) {
+            a.otw2d = 1;
+            st.hi_off = trial.add_pass_table(Ns, Lq);
+        } else {
+            int shift = 0;
+            while ((int64_t(1) << (2 * shift)) < M) ++shift;
+            a.otw_shift = shift;
+            st.lo_off = trial.add_linear(int64_t(1) << shift, M, 1);
+            st.hi_off = trial.add_linear(ceil_div(M, int64_t(1) << shift), M, int64_t(1) << shift);
+        }
+    }
+    tb = trial;
+    a.ip = ip;
+    a.tile = 1;
+    a.tfpc = W;
+    a.tfp = W;
+    a.pshift = ps;
+    a.nbuf = 1;
+    a.wsize = (int32_t)buf;
+    a.spitch = spitch;
+    a.smem_bytes = (int32_t)smem;
+    return true;
+}
+
 // One column pass over an axis of length n (stride S between samples, S
 // independent columns per item, `items` items `D` apart).  The pass runs the
 // q-th factor Lq of the axis decomposition after a product Ns of earlier
@@ -510,7 +710,6 @@ bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64
     st = Step{};
     st.kind = Step::COL;
     ColArgs& a = st.col;
-    if (!build_inner(Lq, rad, nthr, tb, a.ip)) return false;
     a.ncols = items * cpi;
     a.cpi = cpi;
     a.in_dist = D;
@@ -531,86 +730,8 @@ bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64
     a.staged_out = staged_out ? 1 : 0;
     a.scale = 1.f;
     st.tw_off = 0;
-    a.codelet = -1;
-    // plain column passes of a length with a codelet run as column tiles of
-    // that codelet (one transform group per column, in-place passes)
-    if (Ns == 1 && !staged_out && codelets_enabled()) {
-        // the codelet of this length whose launch bound holds 8 to 16
-        // columns with the most threads resident per SM (independent CTAs
-        // overlap one tile's loads with another's passes: 8 columns of 512
-        // points at 3 CTAs per SM ran the strided axes of a 512^3 C2C 10 %
-        // faster than 16 columns at one), then the most columns (wider
-        // tiles read longer row segments); the first such entry on ties
-        // (OPS_FFT_COLTILE_VARIANT=k: the k-th codelet of the length, tiles
-        // of at least 4 columns; tuning experiments)
-        int id = -1, cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
-        const char* env_cv = std::getenv("OPS_FFT_COLTILE_VARIANT");
-        int min_tf = 8;
-        if (env_cv) {
-            const int cand = gfft_codelet_find(Lq, std::atoi(env_cv));
-            if (cand >= 0 && gfft_codelet_info(cand, &cl, &cn, cr, &cnr, &cmaxt, &cminb) == 0 && 4 * cn <= cmaxt) {
-                id = cand;
-                min_tf = 4;
-            }
-        }
-        if (id < 0) {
-            int best_cols = 0, best_res = 0;
-            for (int k = 0;; ++k) {
-                const int cand = gfft_codelet_find(Lq, k);
-                if (cand < 0) break;
-                if (gfft_codelet_info(cand, &cl, &cn, cr, &cnr, &cmaxt, &cminb) != 0) continue;
-                const int cols = std::min(16, cmaxt / cn);
-                const int res = cmaxt * cminb;
-                if (cols >= 8 && (res > best_res || (res == best_res && cols > best_cols))) {
-                    best_cols = cols;
-                    best_res = res;
-                    id = cand;
-                }
-            }
-            if (id >= 0) gfft_codelet_info(id, &cl, &cn, cr, &cnr, &cmaxt, &cminb);
-        }
-        if (id >= 0) {
-            TwiddleBuilder trial = tb;
-            InnerPlan ip;
-            const std::vector<int> crad(cr, cr + cnr);
-            if (build_inner(Lq, crad, cn, trial, ip)) {
-                int64_t lo = -1, hi = -1;
-                for (int p = 0; p < ip.npass; ++p) {
-                    const PassDesc& d = ip.pass[p];
-                    if (d.ns <= 1) continue;
-                    lo = lo < 0 ? d.tw_off : std::min<int64_t>(lo, d.tw_off);
-                    hi = std::max<int64_t>(hi, d.tw_off + (int64_t)d.ns * d.radix);
-                }
-                const int64_t tw_cnt = lo < 0 ? 0 : hi - lo;
-                const int pshift = (cr[0] % 2 == 0) ? 4 : 30;
-                const int64_t wsize = ((int64_t)(Lq - 1) + ((int64_t)(Lq - 1) >> pshift) + 1) | 1;
-                int tfc = 1;
-                while (tfc * 2 * cn <= cmaxt && tfc < 16) tfc *= 2;
-                const int64_t twb = (tw_cnt * 8 + 127) & ~int64_t(127);
-                // up to 72 KB per CTA (several CTAs per SM) when the launch bound
-                // allows more than one CTA per SM; a single-CTA bound takes all
-                const int64_t cap = cminb > 1 ? 72 * 1024 : kMaxSmemBytes;
-                while (tfc > 1 && twb + (int64_t)tfc * wsize * 8 > cap) tfc /= 2;
-                const int64_t smem = twb + (int64_t)tfc * wsize * 8;
-                // tiles narrower than 8 columns (64-byte row segments) lose more to
-                // sector granularity than the in-place passes gain (measured on
-                // 2048-point columns: 2 columns per tile were 1.7x slower than the
-                // column kernel's 4)
-                if (tfc >= min_tf && smem <= kMaxSmemBytes && tw_cnt * 8 <= 64 * 1024) {
-                    tb = trial;
-                    a.ip = ip;
-                    a.codelet = id;
-                    a.tfpc = tfc;
-                    a.tfp = tfc;
-                    a.nbuf = 1;
-                    a.tw_lo = (int32_t)(lo < 0 ? 0 : lo);
-                    a.tw_cnt = (int32_t)tw_cnt;
-                    a.wsize = (int32_t)wsize;
-                    a.smem_bytes = (int32_t)smem;
-                }
-            }
-        }
-    }
+    if (make_tile_col(S, Lq, Ns, staged_out, tb, st)) return true;
+    if (!build_inner(Lq, rad, nthr, tb, a.ip)) return false;
     if (Ns > 1) {
         const int64_t M = Ns * Lq;
         int shift = 0;
@@ -770,8 +891,11 @@ bool build_scratch_c2c_steps(int64_t n, int64_t batch, TwiddleBuilder& tb, std::
     const std::vector<int> fac = split_axis(n, col_max_length());
     if (fac.size() != 2) return false;
     Step first, second;
-    if (!make_col_step(n, 1, batch, n, fac[0], 1, tb, first)) return false;
-    if (!make_col_step(n, 1, batch, n, fac[1], fac[0], tb, second)) return false;
+    t_no_tiles = true;
+    const bool ok = make_col_step(n, 1, batch, n, fac[0], 1, tb, first) &&
+                    make_col_step(n, 1, batch, n, fac[1], fac[0], tb, second);
+    t_no_tiles = false;
+    if (!ok) return false;
     first.src = BUF_IN;
     first.dst = BUF_WS;
     second.src = BUF_WS;

@@ -1,0 +1,127 @@
+"""The register-to-register tile kernel (csrc/tile_fft.cuh) at the sizes where
+it can go wrong: every radix alone and as first, inner and last radix, odd and
+power-of-two paddings, rows and columns that do not fill a tile, one thread
+per row, staged outputs and the outer-twiddle table of long transforms.
+
+Tolerance: a radix-2 level rounds each output twice (one product, one sum), so
+the relative L2 error of log2 N levels stays below 2 * 2^-24 * log2 N."""
+import math
+
+import numpy as np
+import pytest
+
+import aclfft as A
+import oracle as O
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _bound(n):
+    return 2.0 * 2.0 ** -24 * max(math.log2(n), 2.0)
+
+
+def _ok(out, exact, n, what):
+    e = O.errors(out, exact)
+    assert e["rel_l2"] <= _bound(n), (what, e)
+
+
+def _cplx(rng, *shape):
+    return (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)).astype(np.complex64)
+
+
+# (length, rows): single radices, two radices of every kind in both places,
+# three and four passes, the longest row of 512 threads; 1 row, a partly
+# filled tile, more rows than one wave
+ROWS = [(r, 5) for r in range(2, 17)] + [
+    (18, 33), (20, 64), (22, 67), (26, 3), (28, 31), (30, 100), (32, 40000), (36, 7), (60, 1), (64, 1), (64, 70),
+    (105, 9), (143, 4), (154, 300), (180, 2), (210, 1), (224, 17), (420, 50), (1000, 3), (1001, 2), (1155, 2),
+    (1536, 4), (1859, 3), (2310, 301), (3000, 5), (3375, 2), (5040, 2), (6000, 3), (7680, 2)]
+
+
+@pytest.mark.parametrize("n,b", ROWS)
+def test_rows(n, b):
+    rng = np.random.default_rng(n)
+    x = _cplx(rng, b, n)
+    xd = torch.from_numpy(x).cuda()
+    with A.Plan.plan1d(n, A.C2C, b) as p:
+        assert p.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        yd = torch.empty_like(xd)
+        p.exec_c2c(xd, yd, A.FORWARD)
+        zd = xd.clone()
+        p.exec_c2c(zd, zd, A.BACKWARD)  # in place
+    _ok(yd.cpu().numpy(), O.c2c(x, -1), n, ("fwd", n, b))
+    _ok(zd.cpu().numpy(), O.c2c(x, 1), n, ("bwd", n, b))
+
+
+@pytest.mark.parametrize("n,b", [(6, 5), (15, 9), (26, 33), (64, 70), (100, 31), (105, 9), (210, 1), (256 * 7, 3),
+                                 (448, 5), (999, 3), (1001, 2), (2100, 1), (2310, 7), (4620, 3), (6720, 2), (12000, 2)])
+def test_real_rows_and_adjoints(n, b):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((b, n)).astype(np.float32)
+    X = _cplx(rng, b, n // 2 + 1)
+    st = torch.cuda.current_stream()
+    with A.Plan.plan1d(n, A.R2C, b) as p, A.Plan.plan1d(n, A.C2R, b) as q:
+        assert p.check() == "ok" and q.check() == "ok"
+        p.set_stream(st)
+        q.set_stream(st)
+        xd, Xd = torch.from_numpy(x).cuda(), torch.from_numpy(X).cuda()
+        Yd, yd = torch.empty_like(Xd), torch.empty_like(xd)
+        ad, bd = torch.empty_like(xd), torch.empty_like(Xd)
+        p.exec_r2c(xd, Yd)
+        q.exec_c2r(Xd, yd)
+        p.exec_r2c_adjoint(Xd, ad)
+        q.exec_c2r_adjoint(xd, bd)
+    _ok(Yd.cpu().numpy(), O.r2c(x), n, ("r2c", n))
+    _ok(yd.cpu().numpy(), O.c2r(X, n), n, ("c2r", n))
+    w = np.full(n // 2 + 1, 2.0)
+    w[0] = 1
+    if n % 2 == 0:
+        w[-1] = 1
+    _ok(ad.cpu().numpy(), O.c2r((X / w).astype(np.complex128), n), n, ("r2c adjoint", n))
+    _ok(bd.cpu().numpy(), O.r2c(x) * w, n, ("c2r adjoint", n))
+
+
+@pytest.mark.parametrize("b,nx,ny", [(1, 30, 7), (3, 77, 33), (2, 143, 50), (1, 512, 19), (1, 1024, 130), (1, 2048, 66),
+                                     (2, 169, 21), (5, 15, 100), (1, 1859, 12), (1, 16, 5000)])
+def test_columns(b, nx, ny):
+    rng = np.random.default_rng(nx)
+    x = _cplx(rng, b, nx, ny)
+    with A.Plan.plan2d(b, nx, ny) as p:
+        assert p.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        xd = torch.from_numpy(x).cuda()
+        yd = torch.empty_like(xd)
+        p.exec_c2c(xd, yd, A.FORWARD)
+    _ok(yd.cpu().numpy(), np.fft.fft2(x.astype(np.complex128)), nx * ny, (b, nx, ny))
+
+
+# staged first passes (even and odd pass lengths), the outer-twiddle table and,
+# above 2^20 points, the product of two tables
+@pytest.mark.parametrize("n,b", [(14641, 3), (18432, 2), (46200, 5), (45045, 1), (131072, 3), (262144, 1), (1 << 21, 1)])
+def test_long_rows(n, b):
+    rng = np.random.default_rng(n)
+    x = _cplx(rng, b, n)
+    with A.Plan.plan1d(n, A.C2C, b) as p:
+        assert p.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        xd = torch.from_numpy(x).cuda()
+        yd = torch.empty_like(xd)
+        p.exec_c2c(xd, yd, A.BACKWARD)
+    _ok(yd.cpu().numpy(), np.fft.ifft(x.astype(np.complex128), norm="forward"), n, (n, b))
+
+
+def test_columns_longer_than_4_gb():
+    """256 strided samples whose span needs 64-bit offsets; sampled columns."""
+    n, b = 256, (1 << 21) + 3
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    xd = torch.view_as_complex(torch.randn((n, b, 2), generator=g, device="cuda"))
+    cols = torch.tensor([0, 1, 15, 16, 12345, b // 2, b - 17, b - 2, b - 1], device="cuda")
+    want = np.fft.fft(xd[:, cols].cpu().numpy().astype(np.complex128), axis=0)
+    with A.Plan.plan1d(n, A.C2C, b, A.VERTICAL) as p:
+        assert p.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        p.exec_c2c(xd, xd, A.FORWARD)
+    _ok(xd[:, cols].cpu().numpy(), want, n, "wide")
