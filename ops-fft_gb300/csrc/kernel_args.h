@@ -188,63 +188,62 @@ struct TcArgs {
 };
 
 // Ragged batches: many transforms of different lengths and kinds in one
-// persistent launch.  A transform class (one kind and length) owns an
-// on-chip plan; a work item is a group of same-class transforms done on chip
-// (RAG_SINGLE), or one step of a long transform split as n' = L1*L2 (n' = n
-// for C2C, n/2 for even R2C): RAG_P1 (a group of the L2 columns: length-L1
-// transforms of x[j + L2*i] into the workspace), RAG_P2 (a group of the L1
-// rows: twiddled length-L2 transforms from the workspace into the output,
-// or into the second workspace half for R2C) and RAG_POST (even/odd
-// post-process of a long R2C).  P2 items wait until all P1 items of their
-// transform are done, POST items until all P2 items are; items are queued in
-// that order, so every wait is on items already being processed.
-enum RagType : int32_t { RAG_C2C = 0, RAG_R2C = 1 };
-enum RagMode : int32_t { RAG_MODE_SINGLE = 0, RAG_MODE_LONG = 1 };
+// persistent launch.  A work item is a tile of up to 512 threads with up to
+// 16 elements each (csrc/ragged.cu), described by one self-contained record:
+// RAG_SINGLE, a group of same-length transforms done on chip; or one step of
+// a long transform, split as n' = La*Lb (n' = n for C2C and odd R2C, n/2 for
+// even R2C): RAG_P1, a group of the Lb columns: La-point transforms of
+// x[j + Lb*i] to ws[j*La + k]; RAG_P2, a group of the La columns: Lb-point
+// transforms of W_n'^{j*i} ws[j + La*i] to bins j + La*k of the output (of
+// the second workspace half for even R2C); RAG_POST, a range of the even/odd
+// post-process of a long even R2C.  P2 items wait until all P1 items of
+// their transform are done, POST items until all P2 items are; a step is
+// queued after the steps it waits for, so every wait is on items already
+// claimed by running CTAs.
 enum RagItemKind : int32_t { RAG_SINGLE = 0, RAG_P1 = 1, RAG_P2 = 2, RAG_POST = 3 };
-
-struct RagClass {
-    InnerPlan ip;      // single: the whole on-chip transform (length L); long: length L1
-    InnerPlan ip2;     // long: length L2
-    int32_t n;         // transform length
-    int32_t type;      // RagType
-    int32_t mode;      // RagMode
-    int32_t L;         // complex length transformed (n for C2C and odd R2C, n/2 for even R2C)
-    int32_t L1, L2;    // long: L = L1 * L2
-    int32_t group;     // single: transforms per item; long: columns per P1 item
-    int32_t group2;    // long: rows per P2 item
-    int32_t pitch;     // single: shared-memory pitch of one transform (float2)
-    int32_t otw_shift; // long: W_L^{k1*n2} = hi[e >> shift] * lo[e & mask]
-    int64_t post_off;  // even R2C: W_n^k, k <= n/4 + 1 (float2 offset in the blob)
-    int64_t hi_off, lo_off;
-    // pass-table windows [tw_lo, tw_lo + tw_cnt) of ip and ip2, staged in
-    // shared memory after the data buffers at float2 offset tw_smem
-    int64_t tw_lo, tw2_lo;
-    int32_t tw_cnt, tw2_cnt;
-    int32_t tw_smem, tw2_smem;
+enum RagFlags : int32_t {
+    RAG_CONJ_IN = 1,    // conjugate on load when the exec runs backward (C2C)
+    RAG_CONJ_OUT = 2,   // conjugate and scale on store (C2C)
+    RAG_REAL_IN = 4,    // real input (odd R2C)
+    RAG_HALF_OUT = 8,   // keep bins 0..n/2 (odd R2C)
+    RAG_R2C_POST = 16,  // even/odd post-process on chip (even R2C)
+    RAG_WS_OUT = 32,    // P2: bins go to the workspace
 };
-
-struct RagXform {
-    int64_t in_off;   // byte offsets from the exec's input / output pointers
-    int64_t out_off;
-    int64_t ws_off;   // long transforms: float2 offset of its workspace (2*L for R2C, L for C2C)
-    int32_t cls;
-    int32_t pad_;
-};
+constexpr int kRagMaxPass = 8;
 
 struct RagItem {
-    int32_t kind;   // RagItemKind
-    int32_t cls;
-    int32_t first;  // single: index into the order array; P1/P2: first column / row
-    int32_t count;  // transforms / columns / rows in this item
-    int32_t xform;  // P1/P2/POST: the transform
-    int32_t need;   // P2/POST: completed items of the transform to wait for
+    int32_t kind, flags;
+    int32_t L;           // on-chip length (POST: n')
+    int32_t T;           // threads per transform
+    int32_t W;           // transforms per tile
+    int32_t count;       // transforms in this item (POST: pairs)
+    int32_t np;          // passes
+    int32_t ps;          // shared padding: i + (i >> ps)
+    int32_t first;       // SINGLE: first entry of the row table; P1/P2: first column; POST: first pair
+    int32_t xform;       // P1/P2/POST: completion counter
+    int32_t need;        // P2/POST: completed items of the transform to wait for
+    int32_t otw_shift;   // P2: W_n'^e = hi[e >> shift] * lo[e & mask]; -1: one table, e = i*j at hi_off + i*La + j
+    int32_t stride;      // P1/P2: elements between a column's samples
+    int32_t pitch;       // SINGLE: shared pitch of a row; P1: of a staged column
+    uint32_t wmagic;     // thread / (W or T) = thread * wmagic >> 20 (thread < 512)
+    int32_t nhalf;       // odd R2C: n / 2
+    int64_t in_off;      // P1: bytes into the input; P2/POST: float2 into the workspace
+    int64_t out_off;     // P1: float2 into the workspace; P2/POST: bytes into the output (RAG_WS_OUT: float2)
+    int32_t hi_off, lo_off;  // float2 offsets in the twiddle blob
+    int32_t post_off;        // even R2C: W_n^k
+    int32_t pad_;
+    PassDesc pass[kRagMaxPass];
+};
+static_assert(sizeof(RagItem) % 16 == 0, "items are copied in 16-byte units");
+
+// Input and output byte offsets of one row of a RAG_SINGLE item.
+struct RagRow {
+    int64_t in_off, out_off;
 };
 
 struct RagArgs {
-    const RagClass* cls;
-    const RagXform* xf;
-    const int32_t* order;  // single items: transform indices grouped by class
     const RagItem* items;
+    const RagRow* rows;
     int32_t nitems;
     int32_t smem_bytes;
     int32_t ctas;   // persistent CTAs to launch (gfft_ragged_ctas * SM count)

@@ -231,6 +231,8 @@ constexpr int kTileMaxThreads = 512;
 constexpr int kTileElems = 16;  // elements a thread holds
 constexpr int64_t kTileMaxCols = (int64_t(1) << 31) - 64;  // 32-bit column arithmetic
 
+}  // namespace
+
 int tile_threads(int L, const std::vector<int>& rad)
 {
     int t = 1;
@@ -246,7 +248,7 @@ int tile_threads(int L, const std::vector<int>& rad)
 // addresses of a butterfly an arithmetic sequence, the others descending.
 // c2r: the first pass reads the exchange buffer too (the Hermitian
 // pre-process wrote it), so L/R0 has to be a multiple of a power-of-two R0.
-std::vector<int> choose_tile_radices(int L, bool c2r = false)
+std::vector<int> choose_tile_radices(int L, bool c2r, int max_threads)
 {
     if (L == 1) return {1};
     std::vector<int> best, cur;
@@ -255,6 +257,7 @@ std::vector<int> choose_tile_radices(int L, bool c2r = false)
         if ((int)cur.size() > best_np || (int)cur.size() >= kMaxPass) return;
         if (rem == 1) {
             const int np = (int)cur.size(), t = tile_threads(L, cur);
+            if (t > max_threads) return;
             const int mn = *std::min_element(cur.begin(), cur.end());
             if (np < best_np || (np == best_np && (t < best_t || (t == best_t && mn > best_min)))) {
                 best = cur;
@@ -285,13 +288,15 @@ std::vector<int> choose_tile_radices(int L, bool c2r = false)
 }
 
 // log2 of the first radix when that is a power of two: the shared padding
-int tile_pshift(int L, const std::vector<int>& rad, bool c2r = false)
+int tile_pshift(int L, const std::vector<int>& rad, bool c2r)
 {
     if (rad.size() < 2 || (rad[0] & (rad[0] - 1)) != 0 || (c2r && (L / rad[0]) % rad[0])) return 30;
     int s = 0;
     while ((1 << s) < rad[0]) ++s;
     return s;
 }
+
+namespace {
 
 // Score bonus of a codelet configuration with a per-group work buffer
 // (ping-pong passes) over the in-place one.

@@ -3,14 +3,14 @@
 //
 // Plan creation groups the transforms into classes (kind, length), builds
 // each class's on-chip plan - one Stockham transform, or a two-step split
-// L = L1 * L2 for lengths beyond one CTA - and the work-item table the
-// persistent kernel consumes (csrc/ragged.cu).  Item order: the first steps
-// of long transforms, then the on-chip groups by decreasing cost (longest
-// first, so the tail of the launch is short items), then the second steps
-// and post-processes, which wait on counters for the earlier steps.
+// L = La * Lb for lengths beyond one CTA - and the work-item table the
+// persistent kernel consumes (csrc/ragged.cu).  Item order: the long
+// transforms in groups, a group's second steps (which wait on counters for
+// its first steps) one group later, then the on-chip items by decreasing
+// cost, so that the launch ends on short items.
 //
-// Autotuning: per class, candidate radix orders and thread counts are timed
-// in isolation on scratch buffers and the fastest is kept; choices are
+// Autotuning: per class, candidate radix orders are timed in isolation on
+// scratch buffers and the fastest is kept; choices are
 // cached process-wide (and in a text file when OPS_FFT_TUNE_CACHE names
 // one) keyed by (kind, length).
 //
@@ -39,18 +39,40 @@ namespace {
 
 using namespace gfft;
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
 constexpr int kSmemBudget = 110 * 1024;  // per CTA (two CTAs per SM)
-constexpr int kMaxTwWindow = 5120;       // float2 entries of a pass-table window staged in shared memory
 constexpr int kMaxSingle = 4096;         // longest on-chip complex length
 constexpr int64_t kMaxLength = 1 << 24;
+constexpr int kOuterTable = 1 << 16;     // longest length with a whole outer-twiddle table (512 KB)
+constexpr int kPostPairs = 4096;         // bin pairs of one post-process item
+// workspace of one group of long transforms: the next group's first steps
+// are queued between a group's first and second steps, so the workspace in
+// flight is two groups and stays in the L2
+constexpr int64_t kGroupBytes = 24 << 20;
 
-int spad_h(int i) { return i + (i >> 4); }
-int row_pitch(int L) { return spad_h(L - 1) + 2; }
+enum RagType : int { RAG_C2C = 0, RAG_R2C = 1 };
+enum RagMode : int { RAG_MODE_SINGLE = 0, RAG_MODE_LONG = 1 };
 
-struct Variant {
-    std::vector<int> rad;
-    int nthr = 0;
+// One on-chip transform of length L on the tile scheme.
+struct TilePlan {
+    int L = 0, T = 0, ps = 30, np = 0;
+    PassDesc pass[kRagMaxPass] = {};
+    int padded() const { return L + (L >> ps); }
+};
+
+// A transform class: one kind and length.
+struct RagClass {
+    TilePlan p1, p2;   // single: the whole transform (p1); long: La and Lb points
+    int n = 0, type = 0, mode = 0;
+    int L = 0;         // complex length transformed (n for C2C and odd R2C, n/2 for even R2C)
+    int La = 0, Lb = 0;  // long: L = La * Lb
+    int group = 0;     // single: transforms per item; long: columns per P1 item
+    int group2 = 0;    // long: columns per P2 item
+    int pitch = 0;     // single: shared pitch of a row; long: of a staged P1 column
+    int otw_shift = 0;
+    int64_t post_off = -1, hi_off = -1, lo_off = -1;
+    bool even_r2c() const { return type == RAG_R2C && !(n & 1); }
+    bool odd_r2c() const { return type == RAG_R2C && (n & 1); }
 };
 
 bool primes_le_13(int64_t n)
@@ -60,43 +82,34 @@ bool primes_le_13(int64_t n)
     return n == 1;
 }
 
-int nthr_for(int L, const std::vector<int>& rad, int cap)
+// Candidate radix sequences of length L: the tile planner's choice, the row
+// planner's, and the first one's reverse.
+std::vector<std::vector<int>> candidates(int L)
 {
-    int nbf = 1;
-    for (int r : rad) nbf = std::max(nbf, L / r);
-    if (nbf <= cap) return nbf;
-    const int waves = (nbf + cap - 1) / cap;
-    return (nbf + waves - 1) / waves;
+    std::vector<std::vector<int>> out;
+    auto add = [&](const std::vector<int>& r) {
+        if (r.empty() || (int)r.size() > kRagMaxPass || tile_threads(L, r) > kThreads) return;
+        if (*std::max_element(r.begin(), r.end()) > 16) return;
+        if (std::find(out.begin(), out.end(), r) == out.end()) out.push_back(r);
+    };
+    const std::vector<int> base = choose_tile_radices(L, false, kThreads);
+    add(base);
+    add(choose_radices(L));
+    add(std::vector<int>(base.rbegin(), base.rend()));
+    return out;
 }
 
-// Candidate on-chip plans of length L: the planner's radix choice, its
-// reverse, a radix <= 8 factorisation, each with the natural thread count
-// and half of it (two butterflies per thread and pass).
-std::vector<Variant> candidates(int L, int cap)
+TilePlan tile_plan(int L, const std::vector<int>& rad, TwiddleBuilder& tb)
 {
-    std::vector<std::vector<int>> rads;
-    std::vector<int> base = choose_radices(L);
-    if (base.empty()) return {};
-    rads.push_back(base);
-    std::vector<int> rev(base.rbegin(), base.rend());
-    if (rev != base) rads.push_back(rev);
-    {
-        std::vector<int> small;
-        int rem = L;
-        for (int r : {8, 4, 2, 7, 5, 3, 13, 11})
-            while (rem % r == 0 && (int)small.size() < kMaxPass) {
-                small.push_back(r);
-                rem /= r;
-            }
-        if (rem == 1 && !small.empty() && small != base && small != rev) rads.push_back(small);
-    }
-    std::vector<Variant> out;
-    for (auto& r : rads) {
-        const int t = nthr_for(L, r, cap);
-        out.push_back({r, t});
-        if (t >= 64 && t % 2 == 0) out.push_back({r, t / 2});
-    }
-    return out;
+    TilePlan t;
+    InnerPlan ip;
+    if (!build_inner(L, rad, 1, tb, ip) || ip.npass > kRagMaxPass) return t;
+    t.L = L;
+    t.T = tile_threads(L, rad);
+    t.ps = tile_pshift(L, rad);
+    t.np = ip.npass;
+    for (int q = 0; q < t.np; ++q) t.pass[q] = ip.pass[q];
+    return t;
 }
 
 struct Key {
@@ -134,8 +147,7 @@ void save_tune_file()
 
 struct ClassPlan {
     RagClass dev{};
-    std::vector<Variant> cand1, cand2;
-    std::vector<InnerPlan> ip1, ip2;  // per candidate
+    std::vector<TilePlan> cand1, cand2;
     Choice choice;
     bool tuned = false;
     std::vector<int> members;  // transform indices
@@ -148,8 +160,10 @@ struct aclfftRaggedPlan_t {
     std::vector<int> len, type;
     std::vector<int64_t> in_off, out_off;
     std::vector<ClassPlan> classes;
-    std::vector<RagXform> xf;
-    std::vector<int32_t> order;
+    std::vector<int> cls;         // class of each transform
+    std::vector<int64_t> ws_off;  // long transforms: float2 offset of their workspace
+    std::vector<RagRow> rows;     // the rows of the single items, in item order
+    std::vector<int> row_xf;      // their transforms
     std::vector<RagItem> items;
     TwiddleBuilder tb;
     int64_t ws_floats2 = 0;
@@ -166,9 +180,7 @@ struct aclfftRaggedPlan_t {
     bool dev_ready = false;
     int device = -1;
     void* tw = nullptr;
-    RagClass* d_cls = nullptr;
-    RagXform* d_xf = nullptr;
-    int32_t* d_order = nullptr;
+    RagRow* d_rows = nullptr;
     RagItem* d_items = nullptr;
     int* d_queue = nullptr;
     int* d_err = nullptr;
@@ -187,15 +199,12 @@ void free_device(aclfftRaggedPlan_t* p)
 {
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     if (p->s_cap) cudaStreamDestroy(p->s_cap);
-    for (void* q : {(void*)p->tw, (void*)p->d_cls, (void*)p->d_xf, (void*)p->d_order, (void*)p->d_items,
-                    (void*)p->d_queue, (void*)p->d_err, (void*)p->d_ws})
+    for (void* q : {(void*)p->tw, (void*)p->d_rows, (void*)p->d_items, (void*)p->d_queue, (void*)p->d_err, (void*)p->d_ws})
         if (q) cudaFree(q);
     p->gexec = nullptr;
     p->s_cap = nullptr;
     p->tw = nullptr;
-    p->d_cls = nullptr;
-    p->d_xf = nullptr;
-    p->d_order = nullptr;
+    p->d_rows = nullptr;
     p->d_items = nullptr;
     p->d_queue = nullptr;
     p->d_err = nullptr;
@@ -215,66 +224,31 @@ void drop_graph(aclfftRaggedPlan_t* p)
     p->g_inv = -1;
 }
 
-// Shared memory an item of the class needs with the chosen variants: the
-// data buffers, then the staged pass-table window.
+// Shared memory an item of the class needs with the chosen variants: one
+// exchange buffer, for P1 also the staged columns.
 int class_smem(const RagClass& c)
 {
-    if (c.mode == RAG_MODE_SINGLE) return (2 * c.group * c.pitch + c.tw_cnt) * 8;
-    const int p1 = (2 * c.L1 * (c.group + 1) + c.tw_cnt) * 8;
-    const int p2 = (2 * c.group2 * c.pitch + c.tw2_cnt) * 8;
-    return std::max(p1, p2);
+    if (c.mode == RAG_MODE_SINGLE) return c.group * c.pitch * 8;
+    return std::max({c.group * c.p1.padded(), c.group * c.pitch, c.group2 * c.p2.padded()}) * 8;
 }
 
-// Contiguous range of the twiddle blob used by an on-chip plan's passes
-// (cnt = 0 when it is too wide to stage).
-void tw_window(const InnerPlan& ip, int64_t& lo, int32_t& cnt)
-{
-    int64_t a = -1, b = -1;
-    for (int q = 0; q < ip.npass; ++q) {
-        const PassDesc& d = ip.pass[q];
-        if (d.ns <= 1) continue;
-        a = a < 0 ? d.tw_off : std::min<int64_t>(a, d.tw_off);
-        b = std::max<int64_t>(b, d.tw_off + (int64_t)d.ns * d.radix);
-    }
-    lo = a < 0 ? 0 : a;
-    cnt = (a < 0 || b - a > kMaxTwWindow) ? 0 : (int32_t)(b - a);
-}
-
-// Applies candidate choice ch to the class's device descriptor.
+// Applies candidate choice ch to the class's plan.
 bool apply_choice(ClassPlan& cp, Choice ch)
 {
     RagClass& c = cp.dev;
-    if (ch.v1 < 0 || ch.v1 >= (int)cp.ip1.size()) return false;
-    c.ip = cp.ip1[ch.v1];
-    tw_window(c.ip, c.tw_lo, c.tw_cnt);
-    c.tw2_lo = 0;
-    c.tw2_cnt = 0;
-    const int budget = kSmemBudget / 8;  // float2 entries
+    if (ch.v1 < 0 || ch.v1 >= (int)cp.cand1.size()) return false;
+    c.p1 = cp.cand1[ch.v1];
     if (c.mode == RAG_MODE_SINGLE) {
-        c.pitch = row_pitch(c.L);
-        int g = std::max(1, kThreads / c.ip.nthr);
-        while (g > 1 && 2 * g * c.pitch + c.tw_cnt > budget) --g;
-        if (2 * g * c.pitch + c.tw_cnt > budget) c.tw_cnt = 0;
-        c.group = g;
+        c.pitch = c.p1.padded() + 1;
+        while (c.p1.T < 16 && c.pitch % 16 != c.p1.T % 16) ++c.pitch;
+        c.group = std::max(1, std::min(kThreads / c.p1.T, kSmemBudget / (c.pitch * 8)));
         c.group2 = 0;
-        c.tw_smem = 2 * g * c.pitch;
     } else {
-        if (ch.v2 < 0 || ch.v2 >= (int)cp.ip2.size()) return false;
-        c.ip2 = cp.ip2[ch.v2];
-        tw_window(c.ip2, c.tw2_lo, c.tw2_cnt);
-        int g = std::max(1, kThreads / c.ip.nthr);
-        g = std::min(g, c.L2);
-        while (g > 1 && 2 * c.L1 * (g + 1) + c.tw_cnt > budget) --g;
-        if (2 * c.L1 * (g + 1) + c.tw_cnt > budget) c.tw_cnt = 0;
-        c.group = g;
-        c.tw_smem = 2 * c.L1 * (g + 1);
-        c.pitch = row_pitch(c.L2);
-        int g2 = std::max(1, kThreads / c.ip2.nthr);
-        g2 = std::min(g2, c.L1);
-        while (g2 > 1 && 2 * g2 * c.pitch + c.tw2_cnt > budget) --g2;
-        if (2 * g2 * c.pitch + c.tw2_cnt > budget) c.tw2_cnt = 0;
-        c.group2 = g2;
-        c.tw2_smem = 2 * g2 * c.pitch;
+        if (ch.v2 < 0 || ch.v2 >= (int)cp.cand2.size()) return false;
+        c.p2 = cp.cand2[ch.v2];
+        c.pitch = c.La | 1;  // consecutive columns in different banks
+        c.group = std::min(kThreads / c.p1.T, c.Lb);
+        c.group2 = std::min(kThreads / c.p2.T, c.La);
     }
     cp.choice = ch;
     return class_smem(c) <= kSmemBudget;
@@ -282,55 +256,101 @@ bool apply_choice(ClassPlan& cp, Choice ch)
 
 double class_cost(const RagClass& c) { return (double)c.L * std::log2((double)std::max(c.L, 2)); }
 
+RagItem tile_item(int kind, const TilePlan& t, int W, int count, int first)
+{
+    RagItem it{};
+    it.kind = kind;
+    it.L = t.L;
+    it.T = t.T;
+    it.W = W;
+    it.count = count;
+    it.np = t.np;
+    it.ps = t.ps;
+    it.first = first;
+    const int d = kind == RAG_SINGLE ? t.T : W;
+    it.wmagic = (uint32_t)(((1 << 20) + d - 1) / d);
+    for (int q = 0; q < t.np; ++q) it.pass[q] = t.pass[q];
+    return it;
+}
+
 void build_items(aclfftRaggedPlan_t* p)
 {
     p->items.clear();
-    p->order.clear();
-    std::vector<RagItem> p1, single, p2, post;
+    p->rows.clear();
+    p->row_xf.clear();
     std::vector<std::pair<double, RagItem>> singles;
-    std::vector<int> np1(p->count, 0), np2(p->count, 0);
+    struct Long {
+        std::vector<RagItem> p1, p2, post;
+    };
+    std::vector<Long> groups(1);
+    int64_t group_bytes = 0;
     for (int ci = 0; ci < (int)p->classes.size(); ++ci) {
         ClassPlan& cp = p->classes[ci];
         const RagClass& c = cp.dev;
+        const int c2c = c.type == RAG_C2C ? RAG_CONJ_IN : 0;
         if (c.mode == RAG_MODE_SINGLE) {
             for (size_t i = 0; i < cp.members.size(); i += c.group) {
-                RagItem it{};
-                it.kind = RAG_SINGLE;
-                it.cls = ci;
-                it.first = (int)p->order.size();
-                it.count = (int)std::min<size_t>(c.group, cp.members.size() - i);
-                for (int k = 0; k < it.count; ++k) p->order.push_back(cp.members[i + k]);
-                singles.push_back({class_cost(c) * it.count, it});
+                const int count = (int)std::min<size_t>(c.group, cp.members.size() - i);
+                RagItem it = tile_item(RAG_SINGLE, c.p1, c.group, count, (int)p->rows.size());
+                it.pitch = c.pitch;
+                it.flags = c2c ? RAG_CONJ_IN | RAG_CONJ_OUT : (c.odd_r2c() ? RAG_REAL_IN | RAG_HALF_OUT : RAG_R2C_POST);
+                it.nhalf = c.n / 2;
+                it.post_off = (int32_t)c.post_off;
+                for (int k = 0; k < count; ++k) {
+                    const int x = cp.members[i + k];
+                    p->rows.push_back({p->in_off[x], p->out_off[x]});
+                    p->row_xf.push_back(x);
+                }
+                singles.push_back({class_cost(c) * count, it});
             }
-        } else {
-            for (int x : cp.members) {
-                for (int j = 0; j < c.L2; j += c.group) {
-                    RagItem it{};
-                    it.kind = RAG_P1;
-                    it.cls = ci;
-                    it.first = j;
-                    it.count = std::min(c.group, c.L2 - j);
-                    it.xform = x;
-                    p1.push_back(it);
-                    ++np1[x];
-                }
-                for (int k = 0; k < c.L1; k += c.group2) {
-                    RagItem it{};
-                    it.kind = RAG_P2;
-                    it.cls = ci;
-                    it.first = k;
-                    it.count = std::min(c.group2, c.L1 - k);
-                    it.xform = x;
-                    p2.push_back(it);
-                    ++np2[x];
-                }
-                if (c.type == RAG_R2C && !(c.n & 1)) {
-                    RagItem it{};
-                    it.kind = RAG_POST;
-                    it.cls = ci;
-                    it.xform = x;
-                    post.push_back(it);
-                }
+            continue;
+        }
+        for (int x : cp.members) {
+            const int64_t bytes = (c.even_r2c() ? 2 : 1) * (int64_t)c.L * 8;
+            if (group_bytes > 0 && group_bytes + bytes > kGroupBytes) {
+                groups.emplace_back();
+                group_bytes = 0;
+            }
+            group_bytes += bytes;
+            Long& g = groups.back();
+            const int64_t ws = p->ws_off[x];
+            int np1 = 0, np2 = 0;
+            for (int j = 0; j < c.Lb; j += c.group, ++np1) {
+                RagItem it = tile_item(RAG_P1, c.p1, c.group, std::min(c.group, c.Lb - j), j);
+                it.xform = x;
+                it.pitch = c.pitch;
+                it.flags = c2c | (c.odd_r2c() ? RAG_REAL_IN : 0);
+                it.stride = c.Lb;
+                it.in_off = p->in_off[x];
+                it.out_off = ws;
+                g.p1.push_back(it);
+            }
+            for (int j = 0; j < c.La; j += c.group2, ++np2) {
+                RagItem it = tile_item(RAG_P2, c.p2, c.group2, std::min(c.group2, c.La - j), j);
+                it.xform = x;
+                it.need = np1;
+                it.flags = c2c ? RAG_CONJ_OUT : (c.odd_r2c() ? RAG_HALF_OUT : RAG_WS_OUT);
+                it.nhalf = c.n / 2;
+                it.stride = c.La;
+                it.in_off = ws;
+                it.out_off = c.even_r2c() ? ws + c.L : p->out_off[x];
+                it.otw_shift = c.otw_shift;
+                it.hi_off = (int32_t)c.hi_off;
+                it.lo_off = (int32_t)c.lo_off;
+                g.p2.push_back(it);
+            }
+            for (int k = 0; c.even_r2c() && k <= c.L / 2; k += kPostPairs) {
+                RagItem it{};
+                it.kind = RAG_POST;
+                it.L = c.L;
+                it.xform = x;
+                it.need = np1 + np2;
+                it.first = k;
+                it.count = std::min(kPostPairs, c.L / 2 + 1 - k);
+                it.in_off = ws + c.L;
+                it.out_off = p->out_off[x];
+                it.post_off = (int32_t)c.post_off;
+                g.post.push_back(it);
             }
         }
     }
@@ -338,12 +358,17 @@ void build_items(aclfftRaggedPlan_t* p)
                      [](const std::pair<double, RagItem>& a, const std::pair<double, RagItem>& b) {
                          return a.first > b.first;
                      });
-    for (auto& it : p2) it.need = np1[it.xform];
-    for (auto& it : post) it.need = np1[it.xform] + np2[it.xform];
-    p->items.insert(p->items.end(), p1.begin(), p1.end());
+    auto put = [&](const std::vector<RagItem>& v) { p->items.insert(p->items.end(), v.begin(), v.end()); };
+    // group g's second steps one group after its first steps, its
+    // post-process one more later; the on-chip items last, longest first, so
+    // that the launch ends on short ones
+    const size_t ng = groups.size();
+    for (size_t g = 0; g < ng + 2; ++g) {
+        if (g < ng) put(groups[g].p1);
+        if (g >= 1 && g - 1 < ng) put(groups[g - 1].p2);
+        if (g >= 2) put(groups[g - 2].post);
+    }
     for (auto& s : singles) p->items.push_back(s.second);
-    p->items.insert(p->items.end(), p2.begin(), p2.end());
-    p->items.insert(p->items.end(), post.begin(), post.end());
     p->smem = 16;
     for (auto& cp : p->classes) p->smem = std::max(p->smem, class_smem(cp.dev));
 }
@@ -368,10 +393,7 @@ bool upload(T*& d, const std::vector<T>& h)
 
 bool upload_tables(aclfftRaggedPlan_t* p)
 {
-    std::vector<RagClass> cls;
-    for (auto& cp : p->classes) cls.push_back(cp.dev);
-    return upload(p->d_cls, cls) && upload(p->d_xf, p->xf) && upload(p->d_order, p->order) &&
-           upload(p->d_items, p->items);
+    return upload(p->d_rows, p->rows) && upload(p->d_items, p->items);
 }
 
 aclfftResult device_setup(aclfftRaggedPlan_t* p)
@@ -440,9 +462,7 @@ RagArgs make_args(aclfftRaggedPlan_t* p, const RagItem* items, int nitems, int s
                   bool inverse)
 {
     RagArgs a{};
-    a.cls = p->d_cls;
-    a.xf = p->d_xf;
-    a.order = p->d_order;
+    a.rows = p->d_rows;
     a.items = items;
     a.nitems = nitems;
     a.smem_bytes = smem;
@@ -480,7 +500,7 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
     auto trial_m = [&](const RagClass& c) { return (int)std::min<int64_t>(2048, std::max<int64_t>(4, kTrialPoints / c.n)); };
     auto ws_per = [](const RagClass& c) -> int64_t {
         if (c.mode != RAG_MODE_LONG) return 0;
-        return (c.type == RAG_R2C && !(c.n & 1)) ? 2 * (int64_t)c.L : c.L;
+        return c.even_r2c() ? 2 * (int64_t)c.L : c.L;
     };
     int64_t scratch = 16, wsmax = 1;
     int maxm = 1;
@@ -493,11 +513,9 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
     void *sin = nullptr, *sout = nullptr;
     int* squeue = nullptr;
     float2* sws = nullptr;
-    RagXform* sxf = nullptr;
-    int32_t* sorder = nullptr;
+    RagRow* srows = nullptr;
     RagItem* sitems = nullptr;
-    RagClass* scls = nullptr;
-    size_t cap_xf = 0, cap_order = 0, cap_items = 0, cap_cls = 0;
+    size_t cap_rows = 0, cap_items = 0;
     bool ok = gfft::dev_alloc(&sin, (size_t)scratch) == cudaSuccess && gfft::dev_alloc(&sout, (size_t)scratch) == cudaSuccess &&
               cudaMemset(sin, 0, (size_t)scratch) == cudaSuccess &&
               gfft::dev_alloc(reinterpret_cast<void**>(&squeue), (size_t)(maxm + 1) * sizeof(int)) == cudaSuccess &&
@@ -519,16 +537,15 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
         // the trial batch: one class (index 0), m transforms packed in scratch
         aclfftRaggedPlan_t tmp;
         tmp.count = m;
-        tmp.xf.resize(m);
+        tmp.in_off.resize(m);
+        tmp.ws_off.resize(m);
         for (int k = 0; k < m; ++k) {
-            RagXform& x = tmp.xf[k];
-            x.in_off = (int64_t)k * ((int64_t)cp.dev.n + 2) * 8;
-            x.out_off = x.in_off;
-            x.ws_off = (int64_t)k * ws_per(cp.dev);
-            x.cls = 0;
+            tmp.in_off[k] = (int64_t)k * ((int64_t)cp.dev.n + 2) * 8;
+            tmp.ws_off[k] = (int64_t)k * ws_per(cp.dev);
         }
+        tmp.out_off = tmp.in_off;
         double best = 1e30;
-        Choice bestc = cp.choice;
+        Choice bestc;
         for (int a1 = 0; a1 < n1 && ok; ++a1)
             for (int a2 = 0; a2 < n2 && ok; ++a2) {
                 if (!apply_choice(cp, {a1, a2})) continue;
@@ -536,7 +553,6 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
                 tmp.classes[0].members.resize(m);
                 for (int k = 0; k < m; ++k) tmp.classes[0].members[k] = k;
                 build_items(&tmp);
-                std::vector<RagClass> cls(1, cp.dev);
                 // trial tables: reallocated only when they grow
                 auto put = [&](auto*& d, size_t& cap, const auto& h) {
                     using T = typename std::decay_t<decltype(h)>::value_type;
@@ -550,15 +566,12 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
                     return h.empty() ||
                            cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess;
                 };
-                if (!put(scls, cap_cls, cls) || !put(sxf, cap_xf, tmp.xf) || !put(sorder, cap_order, tmp.order) ||
-                    !put(sitems, cap_items, tmp.items)) {
+                if (!put(srows, cap_rows, tmp.rows) || !put(sitems, cap_items, tmp.items)) {
                     ok = false;
                     break;
                 }
                 RagArgs ra{};
-                ra.cls = scls;
-                ra.xf = sxf;
-                ra.order = sorder;
+                ra.rows = srows;
                 ra.items = sitems;
                 ra.nitems = (int)tmp.items.size();
                 ra.smem_bytes = tmp.smem;
@@ -585,7 +598,9 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
                     if (ok) cudaEventElapsedTime(&ms, e0, e1);
                     if (rep > 0) tbest = std::min(tbest, ms);
                 }
-                if (tbest < best) {
+                // the planner's choice (the first) stays unless another is 5 %
+                // faster: one length alone is not the mixed batch
+                if (tbest < (bestc.v1 == 0 && bestc.v2 == 0 && best < 1e30 ? 0.95 * best : best)) {
                     best = tbest;
                     bestc = {a1, a2};
                 }
@@ -597,8 +612,7 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    for (void* q : {(void*)sin, (void*)sout, (void*)squeue, (void*)sws, (void*)sxf, (void*)sorder, (void*)sitems,
-                    (void*)scls})
+    for (void* q : {(void*)sin, (void*)sout, (void*)squeue, (void*)sws, (void*)srows, (void*)sitems})
         if (q) cudaFree(q);
     if (!ok) {
         cudaGetLastError();
@@ -638,6 +652,69 @@ bool device_pointer(const void* ptr, int dev)
     return at.type == cudaMemoryTypeDevice && (dev < 0 || at.device == dev);
 }
 
+// On-chip plans of a class: one tile, or two factors of at most kMaxSingle
+// points.
+bool plan_class(ClassPlan& cp, TwiddleBuilder& tb, std::map<int, double>& memo)
+{
+    RagClass& c = cp.dev;
+    auto plans = [&](int L) {
+        std::vector<TilePlan> v;
+        for (auto& r : candidates(L)) v.push_back(tile_plan(L, r, tb));
+        return v;
+    };
+    if (c.L <= kMaxSingle) {
+        cp.cand1 = plans(c.L);
+        if (!cp.cand1.empty()) {
+            c.mode = RAG_MODE_SINGLE;
+            return true;
+        }
+    }
+    c.mode = RAG_MODE_LONG;
+    // the factors whose steps cost least: items of W * len points, each
+    // costing its passes plus about 1.5 for its loads and stores (30000 as
+    // 240 x 125 instead of the balanced 200 x 150: five passes either way,
+    // fuller tiles); a negative entry of the memo marks a length without a plan
+    auto cost = [&](int len) {
+        auto it = memo.find(len);
+        if (it != memo.end()) return it->second;
+        const std::vector<int> r = choose_tile_radices(len, false, kThreads);
+        double v = -1;
+        if (!r.empty() && (int)r.size() <= kRagMaxPass) {
+            const int W = kThreads / tile_threads(len, r);
+            v = ((double)r.size() + 1.5) / ((double)W * len);
+        }
+        memo[len] = v;
+        return v;
+    };
+    int Lb = 0;
+    double best = 0;
+    for (int d = 2; (int64_t)d * d <= c.L; ++d) {
+        if (c.L % d || c.L / d > kMaxSingle) continue;
+        const double a = cost(d), b = cost(c.L / d);
+        if (a < 0 || b < 0) continue;
+        if (Lb == 0 || a + b <= best) {
+            best = a + b;
+            Lb = d;
+        }
+    }
+    if (Lb == 0) return false;
+    c.Lb = Lb;
+    c.La = c.L / Lb;
+    cp.cand1 = plans(c.La);
+    cp.cand2 = plans(c.Lb);
+    if (c.L <= kOuterTable) {
+        c.otw_shift = -1;
+        c.hi_off = tb.add_pass_table(c.La, c.Lb);
+        return true;
+    }
+    int sh = 0;
+    while ((int64_t(1) << (2 * sh)) < c.L) ++sh;
+    c.otw_shift = sh;
+    c.hi_off = tb.add_linear(((c.L - 1) >> sh) + 1, c.L, int64_t(1) << sh);
+    c.lo_off = tb.add_linear(int64_t(1) << sh, c.L, 1);
+    return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -670,8 +747,10 @@ ACLFFT_API aclfftResult aclfftRaggedPlanCreate(aclfftRaggedPlan* plan, int count
     p->in_off.assign(inOffsets, inOffsets + count);
     p->out_off.assign(outOffsets, outOffsets + count);
     p->type.resize(count);
-    p->xf.resize(count);
+    p->cls.resize(count);
+    p->ws_off.resize(count);
     std::map<Key, int> cidx;
+    std::map<int, double> memo;
     for (int i = 0; i < count; ++i) {
         const int t = types[i] == ACLFFT_C2C ? RAG_C2C : RAG_R2C;
         p->type[i] = t;
@@ -689,48 +768,13 @@ ACLFFT_API aclfftResult aclfftRaggedPlanCreate(aclfftRaggedPlan* plan, int count
             c.L = (t == RAG_R2C && !(n & 1)) ? n / 2 : n;
             c.post_off = -1;
             c.hi_off = c.lo_off = -1;
-            if (c.L <= kMaxSingle) {
-                c.mode = RAG_MODE_SINGLE;
-                cp.cand1 = candidates(c.L, kThreads);
-            } else {
-                c.mode = RAG_MODE_LONG;
-                // L1 <= L2: the column step (strided) is the shorter one
-                int L1 = 1;
-                for (int d = 2; (int64_t)d * d <= c.L; ++d)
-                    if (c.L % d == 0) L1 = d;
-                c.L1 = L1;
-                c.L2 = c.L / L1;
-                if (c.L2 > kMaxSingle || c.L1 < 2) {
-                    delete p;
-                    gfft::set_last_error("ragged batches: length does not split into two on-chip factors");
-                    return ACLFFT_NOT_SUPPORTED;
-                }
-                cp.cand1 = candidates(c.L1, kThreads);
-                cp.cand2 = candidates(c.L2, kThreads);
-                int sh = 0;
-                while ((int64_t(1) << (2 * sh)) < c.L) ++sh;
-                c.otw_shift = sh;
-                c.hi_off = p->tb.add_linear(((c.L - 1) >> sh) + 1, c.L, int64_t(1) << sh);
-                c.lo_off = p->tb.add_linear(int64_t(1) << sh, c.L, 1);
+            if (!plan_class(cp, p->tb, memo)) {
+                delete p;
+                gfft::set_last_error("ragged batches: length does not split into two on-chip factors");
+                return ACLFFT_NOT_SUPPORTED;
             }
-            if (t == RAG_R2C && !(n & 1)) c.post_off = p->tb.add_linear(c.L / 2 + 1, n, 1);
-            for (auto& v : cp.cand1) {
-                InnerPlan ip;
-                if (!build_inner(c.mode == RAG_MODE_SINGLE ? c.L : c.L1, v.rad, v.nthr, p->tb, ip)) {
-                    delete p;
-                    return ACLFFT_INTERNAL_ERROR;
-                }
-                cp.ip1.push_back(ip);
-            }
-            for (auto& v : cp.cand2) {
-                InnerPlan ip;
-                if (!build_inner(c.L2, v.rad, v.nthr, p->tb, ip)) {
-                    delete p;
-                    return ACLFFT_INTERNAL_ERROR;
-                }
-                cp.ip2.push_back(ip);
-            }
-            if (cp.ip1.empty() || (c.mode == RAG_MODE_LONG && cp.ip2.empty()) || !apply_choice(cp, {0, 0})) {
+            if (c.even_r2c()) c.post_off = p->tb.add_linear(c.L / 2 + 1, n, 1);
+            if (cp.cand1.empty() || (c.mode == RAG_MODE_LONG && cp.cand2.empty()) || !apply_choice(cp, {0, 0})) {
                 delete p;
                 gfft::set_last_error("ragged batches: no on-chip plan for a length");
                 return ACLFFT_NOT_SUPPORTED;
@@ -740,21 +784,24 @@ ACLFFT_API aclfftResult aclfftRaggedPlanCreate(aclfftRaggedPlan* plan, int count
             ci = f->second;
         }
         p->classes[ci].members.push_back(i);
-        RagXform& x = p->xf[i];
-        x.in_off = inOffsets[i];
-        x.out_off = outOffsets[i];
-        x.cls = ci;
-        x.ws_off = -1;
+        p->cls[i] = ci;
+        p->ws_off[i] = -1;
         const RagClass& c = p->classes[ci].dev;
         if (c.mode == RAG_MODE_LONG) {
-            ++p->nlong;
-            x.ws_off = p->ws_floats2;
-            p->ws_floats2 += (t == RAG_R2C && !(n & 1)) ? 2 * (int64_t)c.L : c.L;
+            // 128-byte aligned: contiguous blocks are written 16 bytes a thread
+            p->ws_off[i] = p->ws_floats2;
+            p->ws_floats2 += ((c.even_r2c() ? 2 : 1) * (int64_t)c.L + 15) / 16 * 16;
         }
+        if (c.L > kMaxSingle) ++p->nlong;
         const int64_t in_b = t == RAG_C2C ? (int64_t)n * 8 : (int64_t)n * 4;
         const int64_t out_b = t == RAG_C2C ? (int64_t)n * 8 : ((int64_t)n / 2 + 1) * 8;
         p->in_min = std::max(p->in_min, (int64_t)inOffsets[i] + in_b);
         p->out_min = std::max(p->out_min, (int64_t)outOffsets[i] + out_b);
+    }
+    if (p->tb.count > 0x7fffffff) {  // 32-bit table offsets in the items
+        delete p;
+        gfft::set_last_error("ragged batches: twiddle tables too large");
+        return ACLFFT_NOT_SUPPORTED;
     }
     build_items(p);
     *plan = p;
@@ -931,61 +978,102 @@ ACLFFT_API int aclfftRaggedDebugCheck(aclfftRaggedPlan plan, char* msg, int msgl
     };
     if (!plan) return report("no plan", -1);
     const int64_t twn = plan->tb.count;
-    std::vector<int> seen_p1(plan->count, 0), seen_p2(plan->count, 0);
-    for (size_t ii = 0; ii < plan->items.size(); ++ii) {
-        const RagItem& it = plan->items[ii];
-        if (it.cls < 0 || it.cls >= (int)plan->classes.size()) return report("item class", 1);
-        const RagClass& c = plan->classes[it.cls].dev;
-        if (class_smem(c) > plan->smem || plan->smem > kSmemBudget) return report("shared memory", 2);
-        auto tw_ok = [&](const InnerPlan& ip) {
-            for (int q = 0; q < ip.npass; ++q)
-                if (ip.pass[q].tw_off >= 0 && ip.pass[q].tw_off + (int64_t)ip.pass[q].ns * ip.pass[q].radix > twn)
-                    return false;
-            return ip.nthr >= 1 && ip.nthr <= kThreads;
-        };
-        if (!tw_ok(c.ip)) return report("pass tables / threads", 3);
-        if (c.tw_cnt < 0 || c.tw_lo + c.tw_cnt > twn || c.tw2_cnt < 0 || c.tw2_lo + c.tw2_cnt > twn)
-            return report("staged twiddle window", 3);
-        auto window_covers = [](const InnerPlan& ip, int64_t lo, int cnt) {
-            if (cnt == 0) return true;
-            for (int q = 0; q < ip.npass; ++q)
-                if (ip.pass[q].ns > 1 &&
-                    (ip.pass[q].tw_off < lo || ip.pass[q].tw_off + (int64_t)ip.pass[q].ns * ip.pass[q].radix > lo + cnt))
-                    return false;
-            return true;
-        };
-        if (!window_covers(c.ip, c.tw_lo, c.tw_cnt) ||
-            (c.mode == RAG_MODE_LONG && !window_covers(c.ip2, c.tw2_lo, c.tw2_cnt)))
-            return report("staged window misses a pass table", 3);
-        if (c.post_off >= 0 && c.post_off + c.L / 2 + 1 > twn) return report("post table", 3);
-        if (it.kind == RAG_SINGLE) {
-            if (c.group * c.ip.nthr > kThreads || it.count < 1 || it.count > c.group) return report("single group", 4);
-            if (c.pitch < spad_h(c.L - 1) + 1) return report("pitch", 4);
-            if (it.first < 0 || it.first + it.count > (int)plan->order.size()) return report("order range", 4);
-            for (int k = 0; k < it.count; ++k) {
-                const int x = plan->order[it.first + k];
-                if (x < 0 || x >= plan->count || plan->xf[x].cls != it.cls) return report("order entry", 4);
+    std::vector<int> done1(plan->count, 0), done2(plan->count, 0);
+    // bytes of a transform's input and output, columns seen per step
+    auto in_bytes = [&](const RagClass& c) { return (int64_t)c.n * (c.type == RAG_C2C ? 8 : 4); };
+    auto out_bytes = [&](const RagClass& c) { return c.type == RAG_C2C ? (int64_t)c.n * 8 : ((int64_t)c.n / 2 + 1) * 8; };
+    std::vector<int64_t> cols1(plan->count, 0), cols2(plan->count, 0), pairs(plan->count, 0), rows_seen(plan->count, 0);
+    for (const RagItem& it : plan->items) {
+        if (plan->smem > kSmemBudget) return report("shared memory", 2);
+        if (it.kind != RAG_POST) {
+            int64_t ns = 1;
+            if (it.np < 1 || it.np > kRagMaxPass || it.T < 1 || it.W < 1) return report("passes", 3);
+            auto pad = [&](int i) { return i + (i >> it.ps); };
+            for (int q = 0; q < it.np; ++q) {
+                const PassDesc& d = it.pass[q];
+                const int R = d.radix, nbf = it.L / (R > 0 ? R : 1), nb = R >= 16 ? 1 : 16 / (R > 0 ? R : 16);
+                if (R < 1 || R > 16 || it.L % R || d.ns != ns || (int64_t)nb * it.T < nbf) return report("pass", 3);
+                if (ns > 1 && (d.tw_off < 0 || d.tw_off + ns * R > twn)) return report("pass tables", 3);
+                for (int j = 0; j < nbf; ++j) {
+                    const int qq = ns > 1 ? (int)(((uint64_t)(unsigned)j * d.ns_magic) >> 32) : j;
+                    if (qq != j / ns) return report("magic division", 3);
+                    const int i0 = (int)(j / ns * ns * R + j % ns), ws = ns == 1 ? 1 : (int)(ns + (ns >> it.ps));
+                    for (int r = 0; r < R; ++r) {
+                        if (q > 0 && pad(j) + r * (nbf + (nbf >> it.ps)) != pad(j + r * nbf)) return report("read stride", 3);
+                        if (q + 1 < it.np && pad(i0) + r * ws != pad(i0 + r * (int)ns)) return report("write stride", 3);
+                    }
+                }
+                ns *= R;
             }
-        } else {
-            if (it.xform < 0 || it.xform >= plan->count || plan->xf[it.xform].cls != it.cls) return report("xform", 5);
-            const RagXform& x = plan->xf[it.xform];
-            const int64_t wsn = (c.type == RAG_R2C && !(c.n & 1)) ? 2 * (int64_t)c.L : c.L;
-            if (x.ws_off < 0 || x.ws_off + wsn > plan->ws_floats2) return report("workspace", 5);
-            if (c.hi_off < 0 || c.hi_off + ((c.L - 1) >> c.otw_shift) + 1 > twn || c.lo_off + (1 << c.otw_shift) > twn)
-                return report("outer twiddles", 5);
-            if ((int64_t)(c.L1 - 1) * (c.L2 - 1) >= c.L) return report("outer index", 5);
-            if (it.kind == RAG_P1) {
-                if (c.group * c.ip.nthr > kThreads || it.first + it.count > c.L2) return report("p1 range", 6);
-                ++seen_p1[it.xform];
-            } else if (it.kind == RAG_P2) {
-                if (!tw_ok(c.ip2) || c.group2 * c.ip2.nthr > kThreads || it.first + it.count > c.L1)
-                    return report("p2 range", 7);
-                if (seen_p1[it.xform] != it.need) return report("p2 queued before its p1 items", 7);
-                ++seen_p2[it.xform];
-            } else {
-                if (seen_p1[it.xform] + seen_p2[it.xform] != it.need) return report("post queued early", 8);
-            }
+            if (ns != it.L) return report("radix product", 3);
+            if (it.T * it.W > kThreads || it.count < 1 || it.count > it.W) return report("tile threads", 4);
+            const int d = it.kind == RAG_SINGLE ? it.T : it.W;
+            for (int t = 0; t < kThreads; ++t)
+                if ((int)((unsigned)t * it.wmagic >> 20) != t / d) return report("thread division", 4);
+            const int64_t tile = it.kind == RAG_SINGLE ? (int64_t)it.W * it.pitch : (int64_t)it.W * (pad(it.L - 1) + 1);
+            if (tile * 8 > plan->smem || (it.kind == RAG_SINGLE && it.pitch < pad(it.L - 1) + 1))
+                return report("exchange buffer", 4);
         }
+        if (it.kind == RAG_SINGLE) {
+            if (it.first < 0 || it.first + it.count > (int)plan->rows.size()) return report("row range", 4);
+            for (int k = 0; k < it.count; ++k) {
+                const int x = plan->row_xf[it.first + k];
+                const RagClass& c = plan->classes[plan->cls[x]].dev;
+                const RagRow& r = plan->rows[it.first + k];
+                if (c.mode != RAG_MODE_SINGLE || c.L != it.L) return report("row class", 4);
+                if (r.in_off != plan->in_off[x] || r.out_off != plan->out_off[x]) return report("row offsets", 4);
+                if ((it.flags & RAG_R2C_POST) && (it.post_off < 0 || it.post_off + it.L / 2 + 1 > twn))
+                    return report("post table", 4);
+                const int want = c.type == RAG_C2C ? RAG_CONJ_IN | RAG_CONJ_OUT
+                                                   : (c.odd_r2c() ? RAG_REAL_IN | RAG_HALF_OUT : RAG_R2C_POST);
+                if (it.flags != want || it.nhalf != c.n / 2) return report("row mode", 4);
+                ++rows_seen[x];
+            }
+            continue;
+        }
+        if (it.xform < 0 || it.xform >= plan->count) return report("xform", 5);
+        const int x = it.xform;
+        const RagClass& c = plan->classes[plan->cls[x]].dev;
+        const int64_t ws = plan->ws_off[x], wsn = (c.even_r2c() ? 2 : 1) * (int64_t)c.L;
+        if (c.mode != RAG_MODE_LONG || ws < 0 || ws + wsn > plan->ws_floats2) return report("workspace", 5);
+        if (it.kind == RAG_P1) {
+            const int64_t e = (it.flags & RAG_REAL_IN) ? 4 : 8;
+            if (it.L != c.La || it.stride != c.Lb || it.first + it.count > c.Lb) return report("p1 range", 6);
+            if (it.in_off != plan->in_off[x] || (int64_t)c.L * e > in_bytes(c)) return report("p1 input", 6);
+            if (it.out_off != ws) return report("p1 workspace", 6);
+            if (it.pitch < it.L || (int64_t)it.W * it.pitch * 8 > plan->smem) return report("p1 staging", 6);
+            if (done2[x]) return report("p1 queued late", 6);
+            ++done1[x];
+            cols1[x] += it.count;
+        } else if (it.kind == RAG_P2) {
+            if (it.L != c.Lb || it.stride != c.La || it.first + it.count > c.La) return report("p2 range", 7);
+            if (it.need != done1[x] || cols1[x] != c.Lb) return report("p2 queued before its p1 items", 7);
+            if (it.otw_shift < 0 ? it.hi_off < 0 || it.hi_off + (int64_t)c.L > twn
+                                 : it.hi_off < 0 || it.hi_off + ((c.L - 1) >> it.otw_shift) + 1 > twn || it.lo_off < 0 ||
+                                       it.lo_off + (1 << it.otw_shift) > twn || (int64_t)(c.La - 1) * (c.Lb - 1) >= c.L)
+                return report("outer twiddles", 7);
+            if (it.in_off != ws) return report("p2 workspace", 7);
+            const bool wsout = (it.flags & RAG_WS_OUT) != 0;
+            if (wsout != c.even_r2c() || it.out_off != (wsout ? ws + c.L : plan->out_off[x])) return report("p2 output", 7);
+            if (!wsout && !(it.flags & RAG_HALF_OUT) && (int64_t)c.L * 8 > out_bytes(c)) return report("p2 extent", 7);
+            if ((it.flags & RAG_HALF_OUT) && ((int64_t)it.nhalf + 1) * 8 > out_bytes(c)) return report("p2 extent", 7);
+            ++done2[x];
+            cols2[x] += it.count;
+        } else {
+            if (it.need != done1[x] + done2[x] || cols2[x] != c.La) return report("post queued early", 8);
+            if (it.first < 0 || it.count < 1 || it.first + it.count > c.L / 2 + 1 || it.L != c.L || !c.even_r2c())
+                return report("post range", 8);
+            if (it.in_off != ws + c.L || it.out_off != plan->out_off[x] || it.post_off < 0 ||
+                it.post_off + c.L / 2 + 1 > twn)
+                return report("post tables", 8);
+            pairs[x] += it.count;
+        }
+    }
+    for (int x = 0; x < plan->count; ++x) {
+        const RagClass& c = plan->classes[plan->cls[x]].dev;
+        if (c.mode == RAG_MODE_SINGLE ? rows_seen[x] != 1
+                                      : cols1[x] != c.Lb || cols2[x] != c.La || (c.even_r2c() && pairs[x] != c.L / 2 + 1))
+            return report("a transform is not covered once", 9);
     }
     return report("ok", 0);
 }

@@ -125,3 +125,30 @@ def test_columns_longer_than_4_gb():
         p.set_stream(torch.cuda.current_stream())
         p.exec_c2c(xd, xd, A.FORWARD)
     _ok(xd[:, cols].cpu().numpy(), want, n, "wide")
+
+
+# ragged tiles: awkward radix sets (four passes, 11 and 13), tiles that do not
+# divide a factor, outer twiddles as one table (to 2^16) and as a product
+@pytest.mark.parametrize("kind", [A.C2C, A.R2C])
+@pytest.mark.parametrize("lens", [[2, 2, 4, 6, 26, 3146, 4050, 4004, 4095], [4394, 4375, 5005, 8190, 30030, 32760],
+                                  [131072, 148176, 155925, 13 ** 5]])
+def test_ragged_tiles(lens, kind):
+    rng = np.random.default_rng(len(lens))
+    kinds = np.full(len(lens), kind, np.int32)
+    ino, outo, ci, co = A.ragged_layout(lens, kinds)
+    hin = rng.standard_normal(ci // 4).astype(np.float32)
+    din, dout = torch.from_numpy(hin).cuda(), torch.zeros(co // 4, device="cuda")
+    with A.RaggedPlan(np.array(lens, np.int32), kinds, ino, outo) as p:
+        assert p.check() == "ok"
+        p.set_options(autotune=False, graph=False)
+        p.set_stream(torch.cuda.current_stream())
+        p.exec(din, dout, A.FORWARD)
+        assert p.error_flags() == 0
+    hout = dout.cpu().numpy()
+    for n, i, o in zip(lens, ino // 4, outo // 4):
+        if kind == A.C2C:
+            x, y = hin[i:i + 2 * n].view(np.complex64), hout[o:o + 2 * n].view(np.complex64)
+            _ok(y, np.fft.fft(x.astype(np.complex128)), n, ("ragged c2c", n))
+        else:
+            y = hout[o:o + 2 * (n // 2 + 1)].view(np.complex64)
+            _ok(y, np.fft.rfft(hin[i:i + n].astype(np.float64)), n, ("ragged r2c", n))
