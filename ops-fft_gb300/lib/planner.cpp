@@ -446,6 +446,32 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
     return true;
 }
 
+// Whether rows of a length with a compile-time build run on the tile kernel.
+// Measured (us, tile / build): C2C 128 x 131072 42.6 / 110, 256 x 65536 41 /
+// 60, 512 x 32768 47 / 57, 1024 x 16384 44 / 48, 2048 x 8192 46 / 49, 4096 x
+// 4096 51 / 56, but 2048 x 2048 16.6 / 15.9, 4096 x 256 7.5 / 7.1, 512 x 2048
+// 7.5 / 6.8; even real lengths 8192 x 2048 36.7 / 46.6, 512 x 32768 28 / 40,
+// 256 x 65536 31 / 65, but 512 x 2048 5.5 / 4.9, 3000 x 4096 28.7 / 27.0.
+// C2C of 128 and 256 points is faster at every size; below 2^21 points (24
+// MB, where pinned host buffers are used in place, which only the builds do)
+// both gain little.  Adjoints of R2C stay: weighted ones need a build.
+bool tile_beats_codelet(int L, int64_t ntf, int io_mode, int weight)
+{
+    if (std::getenv("OPS_FFT_CODELET_VARIANT")) return false;
+    if (t_hints && (t_hints->codelet_variant >= 0 || t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 ||
+                    t_hints->codelet_pp >= 0))
+        return false;
+    if (weight == WEIGHT_LOAD_HALF) return false;
+    const int64_t points = L * ntf;
+    const bool pow2 = (L & (L - 1)) == 0;
+    switch (io_mode) {
+    case IO_C2C: return pow2 && L <= 4096 && points >= (L <= 256 ? int64_t(1) << 21 : int64_t(1) << 23);
+    case IO_R2C_EVEN:
+    case IO_C2R_EVEN: return pow2 && (L <= 256 || L == 4096) && points >= int64_t(1) << 21;
+    default: return false;
+    }
+}
+
 // Rows of any length with radices <= 16 on the tile kernel.
 bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io_mode, int nreal, int weight,
                         TwiddleBuilder& tb, Step& st)
@@ -519,6 +545,11 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     int maxthr = max_threads_for(rmax);
     int nthr = pick_nthr(L, rad, maxthr);
     int codelet = -1;
+    // large batches of these lengths run faster on the tile kernel although a
+    // compile-time build exists
+    if (tile_beats_codelet(L, ntf, io_mode, weight) &&
+        make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st))
+        return true;
     if (make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
     if (make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
     const bool even_mode = io_mode == IO_R2C_EVEN || io_mode == IO_C2R_EVEN;

@@ -152,3 +152,39 @@ def test_ragged_tiles(lens, kind):
         else:
             y = hout[o:o + 2 * (n // 2 + 1)].view(np.complex64)
             _ok(y, np.fft.rfft(hin[i:i + n].astype(np.float64)), n, ("ragged r2c", n))
+
+
+# lengths with a compile-time build, at the batches where rows move to the
+# tile kernel (and one below)
+@pytest.mark.parametrize("n,b", [(128, 16383), (128, 16384), (256, 8192), (512, 16384), (1024, 8192), (2048, 4096),
+                                 (4096, 2048)])
+def test_rows_of_built_lengths(n, b):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    xd = torch.view_as_complex(torch.randn((b, n, 2), generator=g, device="cuda"))
+    rows = [0, 1, b // 2, b - 2, b - 1]
+    want = np.fft.ifft(xd[rows].cpu().numpy().astype(np.complex128), norm="forward")
+    with A.Plan.plan1d(n, A.C2C, b) as p:
+        assert p.check() == "ok" and (p.info().kernel < 0) == (n * b >= 1 << (21 if n <= 256 else 23))
+        p.set_stream(torch.cuda.current_stream())
+        p.exec_c2c(xd, xd, A.BACKWARD)
+    _ok(xd[rows].cpu().numpy(), want, n, (n, b))
+
+
+@pytest.mark.parametrize("n,b", [(256, 16384), (512, 8192), (8192, 512)])
+def test_real_rows_of_built_lengths(n, b):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    xd = torch.randn((b, n), generator=g, device="cuda")
+    Xd = torch.empty((b, n // 2 + 1), dtype=torch.complex64, device="cuda")
+    yd = torch.empty_like(xd)
+    rows = [0, 1, b // 2, b - 1]
+    with A.Plan.plan1d(n, A.R2C, b) as p, A.Plan.plan1d(n, A.C2R, b) as q:
+        assert p.info().kernel < 0 and q.info().kernel < 0 and p.check() == "ok" and q.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        q.set_stream(torch.cuda.current_stream())
+        p.exec_r2c(xd, Xd)
+        q.exec_c2r(Xd, yd)
+        p.exec_r2c_adjoint_weighted(Xd, torch.ones((b, n // 2 + 1), device="cuda"), torch.empty_like(xd))
+    _ok(Xd[rows].cpu().numpy(), np.fft.rfft(xd[rows].cpu().numpy().astype(np.float64)), n, (n, b))
+    _ok(yd[rows].cpu().numpy(), n * xd[rows].cpu().numpy().astype(np.float64), n * n, (n, b))
