@@ -128,13 +128,19 @@ struct ColArgs {
     // register-to-register tiles of any length with radices <= 16
     // (csrc/tile_fft.cuh): tfpc columns per CTA, exchange buffers (nbuf) of
     // wsize float2, padded by one element every 2^pshift; with otw2d the
-    // outer twiddles come from one table (entry r*ons + j) at otw_hi
+    // outer twiddles W^{j*(jb + r*L/R)} are otw_hi[jb*ons + j] * otw_lo[r*ons + j]
     int32_t tile;
     int32_t wsize;
     int32_t pshift;
     int32_t spitch;  // staged_out: shared pitch of one column
     int32_t otw2d;
-    int32_t pad2_;
+    // IO_C2C, or tiles of paired columns j and pair_m - j: IO_R2C_EVEN, the
+    // last pass of a long even R2C with its post-process, IO_C2R_EVEN, the
+    // first pass of a long even C2R with its pre-process (ncols, cpi: pairs)
+    int32_t io_mode;
+    int32_t pair_m;
+    int32_t weight;
+    const void* post_tw;  // W_N^k, k <= N/2
 };
 
 // Stand-alone even/odd packing for R2C/C2R lengths beyond one CTA.

@@ -18,7 +18,9 @@ int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
     threads = (threads + 31) & ~31;
     if (t.W < 1 || t.ip.nthr < 1 || threads > kTileMaxThreads || t.ncols == 0 || smem > (size_t)kMaxSmemBytes)
         return (int)cudaErrorInvalidValue;
-    const unsigned grid = (t.ncols + (unsigned)t.W - 1) / (unsigned)t.W;
+    const unsigned per = t.rows || !t.M ? (unsigned)t.W : (unsigned)t.W / 2;  // paired columns: two per unit
+    if (per < 1) return (int)cudaErrorInvalidValue;
+    const unsigned grid = (t.ncols + per - 1) / per;
     switch (io) {
     case IO_C2C:
         // the span of one transform decides the offset width
@@ -60,8 +62,6 @@ extern "C" int gfft_launch_tile_row(const RowArgs* a, void* stream)
     t.emul = 1;
     t.cmul = a->lpad;
     t.pshift = a->pshift;
-    t.nbuf = a->nbuf;
-    t.bufsz = a->tfpc * a->lpad;
     t.conj_in = a->conj_in;
     t.conj_out = a->conj_out;
     t.weight = a->weight;
@@ -79,6 +79,7 @@ extern "C" int gfft_launch_tile_col(const ColArgs* a, void* stream)
     if (a->ons > 1) {
         if (a->otw2d) {
             t.otw = static_cast<const float2*>(a->otw_hi);
+            t.otw_lo = static_cast<const float2*>(a->otw_lo);
         } else {
             t.otw_hi = static_cast<const float2*>(a->otw_hi);
             t.otw_lo = static_cast<const float2*>(a->otw_lo);
@@ -110,12 +111,16 @@ extern "C" int gfft_launch_tile_col(const ColArgs* a, void* stream)
     t.emul = a->tfpc;
     t.cmul = 1;
     t.pshift = a->pshift;
-    t.nbuf = a->nbuf;
-    t.bufsz = a->wsize;
     t.staged_out = a->staged_out;
     t.spitch = a->spitch;
     t.conj_in = a->conj_in;
     t.conj_out = a->conj_out;
     t.scale = a->scale;
-    return launch_tile(IO_C2C, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
+    if (a->io_mode != IO_C2C) {
+        t.M = (uint32_t)a->pair_m;
+        t.post = static_cast<const float2*>(a->post_tw);
+        t.weight = a->weight;
+        if (t.M < 1 || !t.post) return (int)cudaErrorInvalidValue;
+    }
+    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
 }

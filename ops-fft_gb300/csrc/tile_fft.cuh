@@ -61,8 +61,11 @@ struct TileArgs {
     InnerPlan ip;
     const float2* tw;
     const float2* post;      // W_N^k, k <= L/2 (even real modes)
-    const float2* otw;       // columns: W_{ons*L}^{i*jm} at i*ons + jm, or nullptr
-    const float2* otw_hi;    // columns: the same as a product of two tables, or nullptr
+    // columns, outer twiddle W_{ons*L}^{jm*i} of sample i = j + r*L/R:
+    // otw[j*ons + jm] * otw_lo[r*ons + jm], or without otw
+    // otw_hi[m >> shift] * otw_lo[m & mask] with m = jm*i, or none
+    const float2* otw;
+    const float2* otw_hi;
     const float2* otw_lo;
     const void* in;
     void* out;
@@ -75,17 +78,19 @@ struct TileArgs {
     int32_t rows;        // 1: rows, 0: columns
     int32_t emul, cmul;  // shared index of element i of transform c: pad(i)*emul + c*cmul
     int32_t pshift;
-    int32_t bufsz;       // float2 per exchange buffer
-    int32_t nbuf;        // exchange buffers (1: one more barrier per inner pass)
-    int32_t staged_out;  // columns: output of column c is out + c*L + k
+    int32_t staged_out;  // columns: the L outputs of a column are contiguous
     int32_t spitch;      // staged_out: shared pitch of one column
+    uint32_t M;          // paired columns: columns of an item (see tile_pair)
     int32_t otw_shift;
     int32_t conj_in, conj_out, weight, nreal;
     float scale;
 };
 
+extern __shared__ __align__(16) float2 tsm[];  // the exchange buffer
+
 struct TileCtx {
     int L, T, tid, ps, em;
+    int off;  // of the transform in the exchange buffer
     bool ok;
     const char* gi;  // the transform's input and output
     char* go;
@@ -115,8 +120,7 @@ __device__ __forceinline__ void tst(void* base, OFF off, float2 x)
 // One pass: radix R, up to 16 / R butterflies per thread, all their inputs
 // in registers before any output is written.
 template <int R, int IO, class OFF, bool FIRST, bool LAST>
-__device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, int p, const float2* src, float2* dst,
-                                          bool mid_sync, bool to_global)
+__device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, int p, bool to_global)
 {
     constexpr int NB = R >= 16 ? 1 : 16 / R;
     const PassDesc& pd = A.ip.pass[p];
@@ -176,15 +180,16 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
                 });
             }
             if (A.otw) {
-                const int64_t ws = (int64_t)nbf * A.ons.d;
                 sfor<NB>([&](auto bb) {
                     constexpr int b = decltype(bb)::value;
                     const int j = c.tid + b * c.T;
                     if (c.ok && j < nbf) {
-                        const float2* w = A.otw + (c.jm + (int64_t)j * A.ons.d);
-                        sfor<R>([&](auto rr) {
-                            constexpr int r = decltype(rr)::value;
-                            v[b * R + r] = cmul(v[b * R + r], ldg2(w + r * ws));
+                        const float2 wa = ldg2(A.otw + c.jm + (int64_t)j * A.ons.d);
+                        const float2* wb = A.otw_lo + c.jm;
+                        v[b * R] = cmul(v[b * R], wa);
+                        sfor<R - 1>([&](auto rr) {
+                            constexpr int r = decltype(rr)::value + 1;
+                            v[b * R + r] = cmul(v[b * R + r], cmul(wa, ldg2(wb + r * A.ons.d)));
                         });
                     }
                 });
@@ -212,13 +217,13 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
             // would be carried around the loop over the passes, for every
             // radix (1.4 KB of stack a thread)
             const int j = min(c.tid + b * c.T, nbf - 1);
-            const float2* s = src + (j + (j >> c.ps)) * c.em;
+            const int s = c.off + (j + (j >> c.ps)) * c.em;
             sfor<R>([&](auto rr) {
                 constexpr int r = decltype(rr)::value;
-                v[b * R + r] = s[r * rs];
+                v[b * R + r] = tsm[s + r * rs];
             });
         });
-        if (mid_sync) __syncthreads();
+        if (!LAST || !to_global) __syncthreads();  // in place: every read precedes any write
     }
     sfor<NB>([&](auto bb) {
         constexpr int b = decltype(bb)::value;
@@ -238,16 +243,16 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
             if (!LAST || !to_global) {
                 int base, ws;
                 if (LAST && A.staged_out) {
-                    base = c.c * A.spitch + j - c.c;  // dst already points at column c
+                    base = c.c * A.spitch + j;
                     ws = ns;
                 } else {
                     const int i0 = q * ns * R + k;
-                    base = (i0 + (i0 >> c.ps)) * c.em;
+                    base = c.off + (i0 + (i0 >> c.ps)) * c.em;
                     ws = (ns == 1 ? 1 : ns + (ns >> c.ps)) * c.em;
                 }
                 sfor<R>([&](auto rr) {
                     constexpr int r = decltype(rr)::value;
-                    dst[base + r * ws] = v[b * R + r];
+                    tsm[base + r * ws] = v[b * R + r];
                 });
             } else if constexpr (IO == IO_R2C_ODD) {
                 const int h = c.L >> 1;
@@ -277,35 +282,54 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
     });
 }
 
-#define GFFT_TILE_CASE(RV, P, FIRST, LAST, DST, MID) \
-    case RV: tile_pass<RV, IO, OFF, FIRST, LAST>(A, c, P, src, DST, MID, direct); break;
-#define GFFT_TILE_SWITCH(P, FIRST, LAST, DST, MID)   \
-    switch (A.ip.pass[P].radix) {                    \
-        GFFT_TILE_CASE(1, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(2, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(3, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(4, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(5, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(6, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(7, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(8, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(9, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(10, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(11, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(12, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(13, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(14, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(15, P, FIRST, LAST, DST, MID) \
-        GFFT_TILE_CASE(16, P, FIRST, LAST, DST, MID) \
-    default: break;                                  \
+#define GFFT_TILE_CASE(RV, P, FIRST, LAST) \
+    case RV: tile_pass<RV, IO, OFF, FIRST, LAST>(A, c, P, direct); break;
+#define GFFT_TILE_SWITCH(P, FIRST, LAST)         \
+    switch (A.ip.pass[P].radix) {                \
+        GFFT_TILE_CASE(1, P, FIRST, LAST) \
+        GFFT_TILE_CASE(2, P, FIRST, LAST) \
+        GFFT_TILE_CASE(3, P, FIRST, LAST) \
+        GFFT_TILE_CASE(4, P, FIRST, LAST) \
+        GFFT_TILE_CASE(5, P, FIRST, LAST) \
+        GFFT_TILE_CASE(6, P, FIRST, LAST) \
+        GFFT_TILE_CASE(7, P, FIRST, LAST) \
+        GFFT_TILE_CASE(8, P, FIRST, LAST) \
+        GFFT_TILE_CASE(9, P, FIRST, LAST) \
+        GFFT_TILE_CASE(10, P, FIRST, LAST) \
+        GFFT_TILE_CASE(11, P, FIRST, LAST) \
+        GFFT_TILE_CASE(12, P, FIRST, LAST) \
+        GFFT_TILE_CASE(13, P, FIRST, LAST) \
+        GFFT_TILE_CASE(14, P, FIRST, LAST) \
+        GFFT_TILE_CASE(15, P, FIRST, LAST) \
+        GFFT_TILE_CASE(16, P, FIRST, LAST) \
+    default: break;                              \
     }
+
+// Columns of the even real modes come in pairs: a tile holds W/2 neighbouring
+// columns u of an item's M and, in its other half, the columns M - u that
+// hold their mirror bins, so the even/odd post-process of the last pass (R2C)
+// and the Hermitian pre-process of the first one (C2R) happen on chip.  The
+// columns 0 and M/2 are their own mirrors and leave theirs empty.
+__device__ __forceinline__ bool tile_pair(const TileArgs& A, uint32_t q, uint32_t& item, uint32_t& u, uint32_t& j)
+{
+    const uint32_t W2 = (uint32_t)A.W >> 1;
+    const uint32_t cu = blockIdx.x * W2 + (q & (W2 - 1));
+    if (cu >= A.ncols) return false;
+    item = tdiv(cu, A.cpi);
+    u = cu - item * A.cpi.d;
+    if (q < W2) {
+        j = u;
+        return true;
+    }
+    j = A.M - u;
+    return u != 0 && 2 * u != A.M;
+}
 
 // OFF: byte offsets within one transform, 32 bits (one add per access) unless
 // its span needs 64 (columns more than 4 GB long).
 template <int MAXT, int MINB, int IO, class OFF = uint32_t>
 __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant__ TileArgs A)
 {
-    extern __shared__ __align__(16) float2 tsm[];
     TileCtx c;
     c.L = A.ip.L;
     c.T = A.ip.nthr;
@@ -321,14 +345,22 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
     const uint32_t c0 = blockIdx.x * (uint32_t)A.W;
     const uint32_t col = c0 + (uint32_t)c.c;
     c.ok = c.c < A.W && c.tid < c.T && col < A.ncols;
+    constexpr bool kEven = IO == IO_R2C_EVEN || IO == IO_C2R_EVEN;
+    uint32_t item = 0, pu = 0, pj = 0;
+    if (kEven && !A.rows) c.ok = tile_pair(A, (uint32_t)c.c, item, pu, pj) && c.tid < c.T;
     if (!c.ok) c.c = 0;
     const uint32_t cl = c.ok ? col : 0u;
     c.jm = 0;
     if (A.rows) {
         c.gi = static_cast<const char*>(A.in) + cl * A.in_dist * (IO == IO_R2C_ODD ? 4 : 8);
         c.go = static_cast<char*>(A.out) + cl * A.out_dist * (IO == IO_C2R_ODD ? 4 : 8);
+    } else if constexpr (kEven) {
+        if (!c.ok) item = pj = 0;
+        c.gi = static_cast<const char*>(A.in) + 8 * (item * A.in_dist + pj);
+        c.go = static_cast<char*>(A.out) + 8 * (item * A.out_dist + pj);
+        c.jm = pj;
     } else {
-        const uint32_t item = tdiv(cl, A.cpi);
+        item = tdiv(cl, A.cpi);
         const uint32_t j = cl - item * A.cpi.d;
         const uint32_t jh = tdiv(j, A.in_split), oh = tdiv(j, A.out_split);
         c.gi = static_cast<const char*>(A.in) + 8 * (item * A.in_dist + jh * A.in_hi + (j - jh * A.in_split.d) * A.in_lo);
@@ -339,15 +371,77 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
         }
     }
     pdl_wait();  // every access below may touch the caller's buffers
-    const int off = c.c * A.cmul;
+    c.off = c.c * A.cmul;
     const int np = A.ip.npass;
     const bool direct = IO != IO_R2C_EVEN && !A.staged_out;  // the last pass stores to HBM
-    float2* src = tsm + off;
-    float2* alt = tsm + (A.nbuf == 2 ? A.bufsz : 0) + off;
     if constexpr (IO == IO_C2R_EVEN) {
         // Hermitian pre-process into the exchange buffer, every bin loaded
         // once (see codelet_kernel); the passes then all run from it
-        if (c.ok) {
+        if (!A.rows) {
+            // column u's samples X[u + r*M] and their mirrors X[L - u - r*M]:
+            // column M - u, sample Lq-1-r (column 0: its own sample Lq-r;
+            // r = 0 pairs DC with Nyquist)
+            const uint32_t W2 = (uint32_t)A.W >> 1;
+            const uint32_t cu = threadIdx.x & (W2 - 1);
+            uint32_t it2 = 0, u = 0, j = 0;
+            if (tile_pair(A, cu, it2, u, j)) {
+                const bool half = A.weight == WEIGHT_LOAD_HALF;
+                const bool self = 2 * u == A.M;
+                const int Lq = c.L, M = (int)A.M;
+                const int rn = u == 0 ? Lq / 2 + 1 : (self ? (Lq + 1) / 2 : Lq);
+                const int n = Lq * M;
+                const float2* x = static_cast<const float2*>(A.in) + it2 * A.in_dist;
+                const int rstep = (int)(blockDim.x / W2);
+                // Z'[i] and Z'[n - i] from X[i] and X[n - i]: with W_N^i for
+                // every i <= n the upper half needs no case of its own
+                auto pre = [&](int r, int rm, uint32_t mo, float2 a, float2 b, float2 w) {
+                    if (half) {
+                        a = cscale(a, 0.5f);
+                        b = cscale(b, 0.5f);
+                    }
+                    const float2 bc = cconj(b);
+                    const float2 ev = cadd(a, bc);
+                    const float2 o = cmulc(csub(a, bc), w);
+                    float2* s0 = tsm + cu;
+                    s0[(r + (r >> c.ps)) * c.em] = cconj(make_float2(ev.x - o.y, ev.y + o.x));
+                    s0[(rm + (rm >> c.ps)) * c.em + mo] = cconj(make_float2(ev.x + o.y, -ev.y + o.x));
+                };
+                int r = (int)(threadIdx.x / W2);
+                if (u != 0 && !self) {
+                    constexpr int U = 4;  // pairs in flight
+                    for (; r + (U - 1) * rstep < Lq; r += U * rstep) {
+                        float2 xa[U], xb[U], w[U];
+                        sfor<U>([&](auto uu) {
+                            constexpr int e = decltype(uu)::value;
+                            const uint32_t i = u + (uint32_t)((r + e * rstep) * M);
+                            xa[e] = tld(x, 8u * i);
+                            xb[e] = tld(x, 8u * (n - i));
+                            w[e] = ldg2(A.post + i);
+                        });
+                        sfor<U>([&](auto uu) {
+                            constexpr int e = decltype(uu)::value;
+                            pre(r + e * rstep, Lq - 1 - r - e * rstep, W2, xa[e], xb[e], w[e]);
+                        });
+                    }
+                    for (; r < Lq; r += rstep) {
+                        const int i = (int)u + r * M;
+                        pre(r, Lq - 1 - r, W2, x[i], x[n - i], ldg2(A.post + i));
+                    }
+                } else {
+                    for (; r < rn; r += rstep) {
+                        const int i = (int)u + r * M;
+                        const float2 a = x[i], b = x[n - i];
+                        if (i == 0) {
+                            tsm[cu] = make_float2(a.x + b.x, -(a.x - b.x));
+                        } else {
+                            // (the middle sample is its own mirror: both stores
+                            // write the same value, W_N^{n/2} = -i)
+                            pre(r, u == 0 ? Lq - r : Lq - 1 - r, 0, a, b, ldg2(A.post + i));
+                        }
+                    }
+                }
+            }
+        } else if (c.ok) {
             const bool half = A.weight == WEIGHT_LOAD_HALF;
             constexpr int U = 4;  // pairs in flight
             for (int k0 = c.tid; k0 <= (c.L >> 1); k0 += U * c.T) {
@@ -364,7 +458,7 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
                     const int k = k0 + u * c.T;
                     if (k == 0) {
                         // imaginary parts of DC and Nyquist ignored
-                        src[0] = make_float2(xa[u].x + xb[u].x, -(xa[u].x - xb[u].x));
+                        tsm[c.off] = make_float2(xa[u].x + xb[u].x, -(xa[u].x - xb[u].x));
                     } else if (k <= (c.L >> 1)) {
                         const int n = c.L - k;
                         float2 a = xa[u], b = xb[u];
@@ -375,70 +469,130 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
                         const float2 bc = cconj(b);
                         const float2 e = cadd(a, bc);
                         const float2 o = cmulc(csub(a, bc), w[u]);
-                        src[k + (k >> c.ps)] = cconj(make_float2(e.x - o.y, e.y + o.x));
-                        if (n != k) src[n + (n >> c.ps)] = cconj(make_float2(e.x + o.y, -e.y + o.x));
+                        tsm[c.off + k + (k >> c.ps)] = cconj(make_float2(e.x - o.y, e.y + o.x));
+                        if (n != k) tsm[c.off + n + (n >> c.ps)] = cconj(make_float2(e.x + o.y, -e.y + o.x));
                     }
                 });
             }
         }
         __syncthreads();
         if (np == 1) {
-            GFFT_TILE_SWITCH(0, false, true, alt, false)
-            return;
+            GFFT_TILE_SWITCH(0, false, true)
+        } else {
+            GFFT_TILE_SWITCH(0, false, false)
         }
-        GFFT_TILE_SWITCH(0, false, false, alt, A.nbuf == 1)
-        __syncthreads();
-        float2* t = src;
-        src = alt;
-        alt = t;
     } else if (np == 1) {
-        GFFT_TILE_SWITCH(0, true, true, src, false)
-        if (!direct) __syncthreads();
+        GFFT_TILE_SWITCH(0, true, true)
     } else {
-        GFFT_TILE_SWITCH(0, true, false, src, false)
-        __syncthreads();
+        GFFT_TILE_SWITCH(0, true, false)
     }
-    if (IO == IO_C2R_EVEN || np > 1) {
+    if (np > 1) {
+        __syncthreads();
         for (int p = 1; p + 1 < np; ++p) {
             // opaque per pass: otherwise every radix' loop-invariant address
             // arithmetic is computed ahead of the loop (40 instructions an
             // element)
             asm volatile("" : "+r"(c.L), "+r"(c.T), "+r"(c.tid), "+r"(c.em), "+r"(c.ps));
-            GFFT_TILE_SWITCH(p, false, false, alt, A.nbuf == 1)
+            GFFT_TILE_SWITCH(p, false, false)
             __syncthreads();
-            float2* t = src;
-            src = alt;
-            alt = t;
         }
-        GFFT_TILE_SWITCH(np - 1, false, true, alt, A.nbuf == 1 && !direct)
-        if (!direct) __syncthreads();
-        src = alt;
+        GFFT_TILE_SWITCH(np - 1, false, true)
     }
-    if constexpr (IO == IO_C2C) {
+    if (direct) return;
+    __syncthreads();
+    if constexpr (IO == IO_C2C || IO == IO_C2R_EVEN) {
         if (A.staged_out) {
-            // the tile's outputs are one contiguous block: consecutive
-            // threads write consecutive bins, two at a time where aligned
-            const float2* s = src - off;
-            float2* g = static_cast<float2*>(A.out) + (int64_t)c0 * c.L;
-            const int ncol = (int)min((uint32_t)A.W, A.ncols - c0);
+            // a column's outputs are contiguous: consecutive threads write
+            // consecutive bins, two at a time where aligned
             const float2 sc = make_float2(A.scale, A.conj_out ? -A.scale : A.scale);
-            if ((reinterpret_cast<uintptr_t>(g) & 15) == 0 && (c.L & 1) == 0) {
-                for (int q = 0; q < ncol; ++q) {
-                    for (int k = 2 * threadIdx.x; k < c.L; k += 2 * blockDim.x) {
-                        const float2 x = pmul(s[q * A.spitch + k], sc), y = pmul(s[q * A.spitch + k + 1], sc);
-                        *reinterpret_cast<float4*>(g + q * c.L + k) = make_float4(x.x, x.y, y.x, y.y);
-                    }
+            const int lane = threadIdx.x & 31;
+            for (int q = threadIdx.x >> 5; q < A.W; q += blockDim.x >> 5) {
+                uint32_t it2 = 0, u = 0, j = 0;
+                if constexpr (IO == IO_C2C) {
+                    if (c0 + q >= A.ncols) break;
+                    it2 = tdiv(c0 + q, A.cpi);
+                    j = c0 + q - it2 * A.cpi.d;
+                } else {
+                    if (!tile_pair(A, (uint32_t)q, it2, u, j)) continue;
                 }
-            } else {
-                for (int q = 0; q < ncol; ++q)
-                    for (int k = threadIdx.x; k < c.L; k += blockDim.x)
-                        g[q * c.L + k] = pmul(s[q * A.spitch + k], sc);
+                float2* g = static_cast<float2*>(A.out) + it2 * A.out_dist + (int64_t)j * c.L;
+                const float2* sq = tsm + q * A.spitch;
+                if ((reinterpret_cast<uintptr_t>(g) & 15) == 0 && (c.L & 1) == 0) {
+#pragma unroll 4
+                    for (int k = 2 * lane; k < c.L; k += 64) {
+                        const float2 x = pmul(sq[k], sc), y = pmul(sq[k + 1], sc);
+                        *reinterpret_cast<float4*>(g + k) = make_float4(x.x, x.y, y.x, y.y);
+                    }
+                } else {
+#pragma unroll 4
+                    for (int k = lane; k < c.L; k += 32) g[k] = pmul(sq[k], sc);
+                }
             }
         }
     }
     if constexpr (IO == IO_R2C_EVEN) {
         // even/odd post-process (see codelet_kernel)
-        if (c.ok) {
+        if (!A.rows) {
+            // bins u + M*kk of column u and their mirrors: column M - u, bin
+            // Lq-1-kk (column 0: its own bin Lq-kk; kk = 0 is DC and Nyquist)
+            const uint32_t W2 = (uint32_t)A.W >> 1;
+            const uint32_t cu = threadIdx.x & (W2 - 1);
+            uint32_t it2 = 0, u = 0, j = 0;
+            if (tile_pair(A, cu, it2, u, j)) {
+                const float sc = A.scale;
+                const float s2 = A.weight == WEIGHT_STORE_X2 ? 2.f * sc : sc;
+                const bool self = 2 * u == A.M;
+                const int Lq = c.L, M = (int)A.M;
+                const int kn = u == 0 ? Lq / 2 + 1 : (self ? (Lq + 1) / 2 : Lq);
+                const int n = Lq * M;
+                float2* out = static_cast<float2*>(A.out) + it2 * A.out_dist;
+                const float2* s = tsm + cu;
+                const int kstep = (int)(blockDim.x / W2);
+                auto post = [&](int k, float2 zk, float2 zn, float2 w) {
+                    const float2 zc = cconj(zn);
+                    const float2 ev = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
+                    const float2 o = make_float2(0.5f * (zk.y - zc.y), 0.5f * (zc.x - zk.x));
+                    const float2 wo = cmul(w, o);
+                    tst(out, 8u * k, cscale(cadd(ev, wo), s2));
+                    if (2 * k != n) tst(out, 8u * (n - k), cscale(cconj(csub(ev, wo)), s2));
+                };
+                int kk = (int)(threadIdx.x / W2);
+                if (u != 0 && !self) {
+                    // with W_N^k for every k <= n the upper half needs no
+                    // case of its own
+                    constexpr int U = 4;  // pairs in flight
+                    for (; kk + (U - 1) * kstep < Lq; kk += U * kstep) {
+                        float2 za[U], zb[U], w[U];
+                        sfor<U>([&](auto uu) {
+                            constexpr int e = decltype(uu)::value;
+                            const int q = kk + e * kstep, m = Lq - 1 - q;
+                            za[e] = s[(q + (q >> c.ps)) * c.em];
+                            zb[e] = s[(m + (m >> c.ps)) * c.em + W2];
+                            w[e] = ldg2(A.post + (u + (uint32_t)(q * M)));
+                        });
+                        sfor<U>([&](auto uu) {
+                            constexpr int e = decltype(uu)::value;
+                            post((int)u + (kk + e * kstep) * M, za[e], zb[e], w[e]);
+                        });
+                    }
+                    for (; kk < Lq; kk += kstep) {
+                        const int m = Lq - 1 - kk, k = (int)u + kk * M;
+                        post(k, s[(kk + (kk >> c.ps)) * c.em], s[(m + (m >> c.ps)) * c.em + W2], ldg2(A.post + k));
+                    }
+                } else {
+                    for (; kk < kn; kk += kstep) {
+                        const int m = u == 0 ? (kk ? Lq - kk : 0) : Lq - 1 - kk, k = (int)u + kk * M;
+                        const float2 zk = s[(kk + (kk >> c.ps)) * c.em], zn = s[(m + (m >> c.ps)) * c.em];
+                        if (k == 0) {
+                            out[0] = make_float2((zk.x + zk.y) * sc, 0.f);
+                            out[n] = make_float2((zk.x - zk.y) * sc, 0.f);
+                        } else {
+                            post(k, zk, zn, ldg2(A.post + k));
+                        }
+                    }
+                }
+            }
+        } else if (c.ok) {
             const float sc = A.scale;
             const float s2 = A.weight == WEIGHT_STORE_X2 ? 2.f * sc : sc;
             constexpr int U = 4;  // pairs in flight
@@ -449,8 +603,8 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
                     const int k = min(k0 + u * c.T, c.L >> 1);
                     const int n = k ? c.L - k : 0;
                     w[u] = ldg2(A.post + k);
-                    za[u] = src[k + (k >> c.ps)];
-                    zb[u] = src[n + (n >> c.ps)];
+                    za[u] = tsm[c.off + k + (k >> c.ps)];
+                    zb[u] = tsm[c.off + n + (n >> c.ps)];
                 });
                 sfor<U>([&](auto uu) {
                     constexpr int u = decltype(uu)::value;

@@ -131,6 +131,7 @@ int launch_list(PlanImpl* impl, const StepList& sl, void* in, void* out, cudaStr
             s.col.tw = tw;
             s.col.otw_hi = s.hi_off >= 0 ? tw + s.hi_off : nullptr;
             s.col.otw_lo = s.lo_off >= 0 ? tw + s.lo_off : nullptr;
+            s.col.post_tw = s.post_off >= 0 ? tw + s.post_off : nullptr;
             s.col.in = src;
             s.col.out = dst;
             if (c2c) {

@@ -202,6 +202,35 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
     const ColArgs& a = s.col;
     if (!check_inner(a.ip, tw_count, why)) return false;
     const int L = a.ip.L;
+    if (a.io_mode != IO_C2C) {
+        // paired columns: whole items on both sides, the packing table, and
+        // the pass that touches bin L
+        const bool r2c = a.io_mode == IO_R2C_EVEN;
+        const int64_t n = (int64_t)L * a.pair_m;
+        if (!a.tile || (!r2c && a.io_mode != IO_C2R_EVEN) || a.tfpc < 2 || (a.tfpc & (a.tfpc - 1)))
+            return fail(why, "paired columns mode");
+        if (a.cpi != a.pair_m / 2 + 1 || a.ncols < 1 || a.ncols % a.cpi || a.ncols * 2 >= (int64_t(1) << 31) - 64)
+            return fail(why, "paired columns");
+        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, !r2c, why)) return false;
+        const int64_t items = a.ncols / a.cpi;
+        if (a.in_stride != a.pair_m || (r2c && a.out_stride != a.pair_m) || (r2c ? a.ons != a.pair_m : a.ons != 1))
+            return fail(why, "paired columns strides");
+        if (a.staged_out != !r2c || (!r2c && (a.spitch < L || (int64_t)a.tfpc * a.spitch > a.wsize)))
+            return fail(why, "paired columns staging");
+        if (a.in_dist < (r2c ? n : n + 1) || a.out_dist < (r2c ? n + 1 : n)) return fail(why, "paired columns rows");
+        if (((items - 1) * a.in_dist + (r2c ? n : n + 1)) * 8 > b.bytes[s.src]) return fail(why, "paired input out of bounds");
+        if (((items - 1) * a.out_dist + (r2c ? n + 1 : n)) * 8 > b.bytes[s.dst]) return fail(why, "paired output out of bounds");
+        if (s.post_off < 0 || s.post_off + n + 1 > tw_count) return fail(why, "paired post table");
+        if (r2c) {
+            const int64_t R0 = a.ip.pass[0].radix;
+            if (a.otw2d ? s.hi_off < 0 || s.hi_off + L / R0 * a.ons > tw_count || s.lo_off < 0 ||
+                              s.lo_off + R0 * a.ons > tw_count
+                        : s.lo_off < 0 || s.lo_off + (int64_t(1) << a.otw_shift) > tw_count || s.hi_off < 0 ||
+                              s.hi_off + (n + (int64_t(1) << a.otw_shift) - 1) / (int64_t(1) << a.otw_shift) > tw_count)
+                return fail(why, "paired outer twiddles");
+        }
+        return true;
+    }
     if (a.tile) {
         if (a.tfpc & (a.tfpc - 1)) return fail(why, "tile column mode");
         if (a.ncols >= (int64_t(1) << 31) - 64) return fail(why, "tile columns");
@@ -221,7 +250,8 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
     if ((in_max + 1) * 8 > b.bytes[s.src]) return fail(why, "col input out of bounds");
     int64_t out_max;
     if (a.staged_out) {
-        out_max = a.ncols * L - 1;
+        // tiles: rows out_dist apart; the column kernel: back to back
+        out_max = a.tile ? (items - 1) * a.out_dist + a.cpi * L - 1 : a.ncols * L - 1;
     } else {
         out_max = (items - 1) * a.out_dist + max_part(a.cpi, a.out_split, a.out_hi, a.out_lo) +
                   (int64_t)(L - 1) * a.out_stride;
@@ -232,7 +262,10 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
         if (M >= (int64_t(1) << 32)) return fail(why, "outer twiddle index overflow");
         if (a.tw_div < 1) return fail(why, "tw_div");
         if (a.otw2d) {
-            if (!a.tile || s.hi_off < 0 || s.hi_off + M > tw_count) return fail(why, "outer twiddle table");
+            const int64_t R0 = a.ip.pass[0].radix;
+            if (!a.tile || s.hi_off < 0 || s.hi_off + L / R0 * a.ons > tw_count || s.lo_off < 0 ||
+                s.lo_off + R0 * a.ons > tw_count)
+                return fail(why, "outer twiddle table");
             return true;
         }
         const int64_t S = int64_t(1) << a.otw_shift;

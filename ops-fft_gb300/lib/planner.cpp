@@ -79,24 +79,26 @@ std::vector<int> choose_radices(int L)
     return best;
 }
 
-int64_t TwiddleBuilder::add_pass_table(int64_t ns, int R)
+int64_t TwiddleBuilder::add_outer(int64_t ns, int64_t rows, int64_t M)
 {
-    // layout [r][k]: entry r*ns + k = W_{ns*R}^{k*r}; consecutive butterflies
-    // (consecutive k) read consecutive entries
+    // layout [row][k]: entry row*ns + k = W_M^{row*k}
     for (const TwSeg& t : segs)
-        if (t.kind == 2 && t.M == ns * R && t.R_or_mult == ns) return t.offset;
+        if (t.kind == 2 && t.M == M && t.R_or_mult == ns && t.count >= rows * ns) return t.offset;
     const int64_t off = count;
     TwSeg s{};
     s.offset = off;
-    s.count = ns * R;
-    s.M = ns * R;
+    s.count = ns * rows;
+    s.M = M;
     s.R_or_mult = ns;
     s.kind = 2;
     segs.push_back(s);
-    count += ns * R;
+    count += ns * rows;
     count += count & 1;
     return off;
 }
+
+// Pass table: consecutive butterflies (consecutive k) read consecutive entries.
+int64_t TwiddleBuilder::add_pass_table(int64_t ns, int R) { return add_outer(ns, R, ns * R); }
 
 int64_t TwiddleBuilder::add_linear(int64_t n, int64_t M, int64_t mult)
 {
@@ -689,12 +691,16 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     if (smem > kMaxSmemBytes) return false;
     if (Ns > 1) {
         const int64_t M = Ns * Lq;
-        // the outer twiddles as one table read like the data (one load an
-        // element, correctly rounded) up to 8 MB, which the L2 holds beside
-        // the data; beyond, the product of two small tables
-        if (M <= (int64_t)1 << 20) {
+        // the outer twiddle W_M^{j*i} of a first-pass butterfly (samples i =
+        // jb + r*Lq/R) is W_M^{j*jb} * W_{Ns*R}^{j*r}: two tables whose rows
+        // of Ns entries are read like the data's, small enough that a tile's
+        // part stays in the L1 (one table of all M entries, read beside the
+        // data, doubled the L2 reads of the pass: 131072 x 128 125 -> 110 us)
+        const int64_t rows = Lq / rad[0];
+        if ((rows + rad[0]) * Ns <= (int64_t)1 << 20) {
             a.otw2d = 1;
-            st.hi_off = trial.add_pass_table(Ns, Lq);
+            st.hi_off = trial.add_outer(Ns, rows, M);
+            st.lo_off = trial.add_pass_table(Ns, rad[0]);
         } else {
             int shift = 0;
             while ((int64_t(1) << (2 * shift)) < M) ++shift;
@@ -713,6 +719,68 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     a.wsize = (int32_t)buf;
     a.spitch = spitch;
     a.smem_bytes = (int32_t)smem;
+    return true;
+}
+
+bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st);
+
+// The two column passes of a long even real transform (complex length L = Lq
+// * Ns) with the even/odd packing on chip: the last pass of an R2C and the
+// first of a C2R run on tiles of paired columns.  Both passes read and write
+// HBM once; the packing as a third pass was a third of the traffic (R2C
+// 262144 x 128 162 -> 149 us, C2R 162 -> 156).  src -> mid -> dst, rows of the
+// middle buffer mid_dist apart.  False when a pass has no tile.
+bool make_pair_steps(int64_t L, int64_t batch, bool r2c, int weight, int src, int mid, int64_t mid_dist, int dst,
+                     const std::vector<int>& fac, TwiddleBuilder& tb, std::vector<Step>& out)
+{
+    TwiddleBuilder trial = tb;
+    const int64_t nb = L + 1;
+    Step a, b;
+    if (!make_col_step(L, 1, batch, L, fac[0], 1, trial, a) || !make_col_step(L, 1, batch, L, fac[1], fac[0], trial, b))
+        return false;
+    if (!a.col.tile || !b.col.tile) return false;
+    // the paired pass: half a tile of neighbouring columns each way (R2C 16
+    // columns, 149 us against 164 with 8; C2R 8, 156 against 160 with 16)
+    Step& ps = r2c ? b : a;
+    ColArgs& c = ps.col;
+    const int Lq = c.ip.L;
+    const std::vector<int> rad = choose_tile_radices(Lq, !r2c);
+    const int T = tile_threads(Lq, rad);
+    int W = r2c ? 16 : 8;
+    while (W > 8 && W * T > kTileMaxThreads) W >>= 1;
+    if (W * T > kTileMaxThreads) return false;
+    if (!build_inner(Lq, rad, T, trial, c.ip)) return false;
+    c.pshift = tile_pshift(Lq, rad, !r2c);
+    c.pair_m = (int32_t)(L / Lq);
+    c.tfpc = W;
+    c.tfp = W;
+    c.io_mode = r2c ? IO_R2C_EVEN : IO_C2R_EVEN;
+    c.weight = weight;
+    c.cpi = c.pair_m / 2 + 1;
+    c.ncols = batch * c.cpi;
+    if (c.ncols * 2 >= kTileMaxCols) return false;
+    c.in_split = c.out_split = c.cpi;
+    int64_t buf = (int64_t)W * (Lq + (Lq >> c.pshift));
+    c.spitch = 0;
+    if (!r2c) {
+        c.spitch = Lq;
+        while (c.spitch % 16 != 16 / W % 16) ++c.spitch;
+        buf = std::max<int64_t>(buf, (int64_t)W * c.spitch);
+    }
+    c.wsize = (int32_t)buf;
+    c.smem_bytes = (int32_t)(buf * 8);
+    if (c.smem_bytes > kMaxSmemBytes) return false;
+    ps.post_off = trial.add_linear(L + 1, 2 * L, 1);
+    a.col.in_dist = r2c ? L : nb;
+    a.col.out_dist = b.col.in_dist = mid_dist;
+    b.col.out_dist = r2c ? nb : L;
+    if (!r2c) b.col.conj_out = 1;
+    a.src = src;
+    a.dst = b.src = mid;
+    b.dst = dst;
+    tb = trial;
+    out.push_back(a);
+    out.push_back(b);
     return true;
 }
 
@@ -1498,7 +1566,17 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
             }
         }
         if (row_ok) return single(mode, (int)L, r2c ? L : nb, r2c ? nb : L);
-        // long real transforms: separate packing around a multi-pass C2C
+        // long real transforms: two passes with the packing on chip; out of
+        // place the middle result sits in the output rows
+        {
+            const std::vector<int> fac = split_axis(L, cap);
+            if (fac.size() == 2 &&
+                make_pair_steps(L, p.batch, r2c, p.weight, IN, BUF_WS, L, BUF_OUT, fac, tb, out.steps)) {
+                need_ws(L * p.batch * 8);
+                return true;
+            }
+        }
+        // longer ones: separate packing around a multi-pass C2C
         Step pk;
         pk.kind = Step::PACK;
         pk.pack.L = (int)L;

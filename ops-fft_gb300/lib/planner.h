@@ -84,6 +84,7 @@ struct TwiddleBuilder {
     std::vector<std::pair<int64_t, int64_t>> dsegs;
     int64_t add_dtable(int64_t n);
     int64_t add_pass_table(int64_t ns, int R);        // rows of R, W_{ns*R}^{k*r}
+    int64_t add_outer(int64_t ns, int64_t rows, int64_t M);  // rows of ns, W_M^{row*k}
     int64_t add_linear(int64_t count, int64_t M, int64_t mult);  // W_M^{i*mult}
     int64_t add_dft_matrix(int R, int prec);  // tensor-core operand images (kind 3)
 };

@@ -188,3 +188,43 @@ def test_real_rows_of_built_lengths(n, b):
         p.exec_r2c_adjoint_weighted(Xd, torch.ones((b, n // 2 + 1), device="cuda"), torch.empty_like(xd))
     _ok(Xd[rows].cpu().numpy(), np.fft.rfft(xd[rows].cpu().numpy().astype(np.float64)), n, (n, b))
     _ok(yd[rows].cpu().numpy(), n * xd[rows].cpu().numpy().astype(np.float64), n * n, (n, b))
+
+
+# paired columns: odd and even pass lengths and column counts on both sides,
+# one item and several, adjoint weights, in place (through the workspace)
+@pytest.mark.parametrize("n,b", [(2 * 14641, 2), (60060, 3), (90090, 1), (92400, 5), (98304, 2), (262144, 3),
+                                 (2 * 15625, 4), (1 << 21, 1)])
+def test_long_real_rows(n, b):
+    rng = np.random.default_rng(n)
+    nb = n // 2 + 1
+    x = rng.standard_normal((b, n)).astype(np.float32)
+    X = _cplx(rng, b, nb)
+    st = torch.cuda.current_stream()
+    w = np.full(nb, 2.0)
+    w[0] = w[-1] = 1
+    xd, Xd = torch.from_numpy(x).cuda(), torch.from_numpy(X).cuda()
+    with A.Plan.plan1d(n, A.R2C, b) as p, A.Plan.plan1d(n, A.C2R, b) as q:
+        assert p.check() == "ok" and q.check() == "ok" and p.info().nsteps == 2
+        p.set_stream(st)
+        q.set_stream(st)
+        Yd, yd, ad, bd = torch.empty_like(Xd), torch.empty_like(xd), torch.empty_like(xd), torch.empty_like(Xd)
+        p.exec_r2c(xd, Yd)
+        q.exec_c2r(Xd, yd)
+        p.exec_r2c_adjoint(Xd, ad)
+        q.exec_c2r_adjoint(xd, bd)
+        ip = torch.zeros(2 * nb * b, device="cuda")
+        ip[:n * b] = xd.reshape(-1)
+        p.exec_r2c(ip, ip)
+        q.set_norm(A.NORM_BACKWARD)
+        p.exec_r2c(xd, Yd)
+        iq = torch.view_as_real(Yd).reshape(-1).clone()
+        q.exec_c2r(iq, iq)
+    assert torch.equal(torch.from_numpy(X).cuda(), Xd)
+    _ok(Yd.cpu().numpy(), np.fft.rfft(x.astype(np.float64)), n, ("r2c", n))
+    assert torch.equal(ip, torch.view_as_real(Yd).reshape(-1))
+    assert torch.all(Yd[:, 0].imag == 0) and torch.all(Yd[:, -1].imag == 0)
+    Xe = X.astype(np.complex128)
+    _ok(yd.cpu().numpy(), n * np.fft.irfft(Xe, n), n, ("c2r", n))
+    _ok(ad.cpu().numpy(), n * np.fft.irfft(Xe / w, n), n, ("r2c adjoint", n))
+    _ok(bd.cpu().numpy(), np.fft.rfft(x.astype(np.float64)) * w, n, ("c2r adjoint", n))
+    _ok(iq[:n * b].cpu().numpy().reshape(b, n), x.astype(np.float64), n * n, ("round trip", n))
