@@ -1,8 +1,9 @@
 // dfft.cu - double-precision (Z2Z / D2Z / Z2D) transforms.
 //
 // GB300's FP64 rate is a small fraction of its FP32 rate, so a
-// double-precision FFT is bound by arithmetic, not by HBM: the passes here
-// are plain global-memory-to-global-memory Stockham passes (one radix-R
+// double-precision FFT is bound by arithmetic, not by HBM: lengths beyond one
+// CTA (csrc/dtile.cu has the others) and radices above 16 run as plain
+// global-memory-to-global-memory Stockham passes (one radix-R
 // butterfly per thread, the same compile-time butterflies as the FP32
 // kernels instantiated on double2), not the shared-memory pipelines of the
 // FP32 path.  A transform of length n = R_1 * ... * R_k is k launches; the
@@ -199,6 +200,7 @@ int launch_r(const DPassArgs* a, cudaStream_t st)
 extern "C" int gfft_launch_dpass(const gfft::DPassArgs* a, void* stream)
 {
     using namespace gfft;
+    if (a->tile) return gfft_launch_dtile(a, stream);
     if (a->n < 1 || a->radix < 1 || a->n % a->radix || a->ns < 1 || (a->n / a->radix) % a->ns || a->ntf < 1 ||
         a->in_split < 1 || a->out_split < 1)
         return (int)cudaErrorInvalidValue;

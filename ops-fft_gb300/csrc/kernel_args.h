@@ -354,14 +354,23 @@ struct DPassArgs {
     int32_t conj_in;   // conjugate on load (backward C2C)
     int32_t conj_out;  // conjugate on store
     int32_t t_fast;    // 1: consecutive threads take consecutive transforms (strided axes)
-    int32_t pad_;
+    // 1: the whole axis in one launch (csrc/dtile.cu): radices in ip (tables
+    // unused), W transforms and `threads` per CTA, shared padding and pitch;
+    // DIO_R2C_POST / DIO_C2R_PRE run on chip with W_2n^k at post
+    int32_t tile;
     double scale;
+    InnerPlan ip;
+    int32_t W, threads, pshift, pitch, smem_bytes;
+    const void* post;
 };
+constexpr int kDTileThreads = 256;  // per CTA, three such CTAs per SM (80 registers)
+constexpr int kDTileElems = 8;  // elements a thread holds (up to 16 for larger radices)
 
 }  // namespace gfft
 
 extern "C" {
 int gfft_launch_dpass(const gfft::DPassArgs* a, void* stream);
+int gfft_launch_dtile(const gfft::DPassArgs* a, void* stream);
 // Fills table[m] = exp(-2 pi i m / n) in FP64 for m < n.
 int gfft_gen_dtwiddles(void* table, long long n, void* stream);
 int gfft_launch_row(const gfft::RowArgs* a, void* stream);

@@ -155,6 +155,7 @@ int launch_list(PlanImpl* impl, const StepList& sl, void* in, void* out, cudaStr
             s.dp.in = src;
             s.dp.out = dst;
             s.dp.tw = tw + s.dtw_off;
+            s.dp.post = s.post_off >= 0 ? tw + s.post_off : nullptr;
             if (c2c) {
                 s.dp.conj_in = first && inverse;
                 s.dp.conj_out = last && inverse;

@@ -347,6 +347,40 @@ bool check_tc(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
 bool check_dpass(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
 {
     const DPassArgs& a = s.dp;
+    if (a.tile) {
+        // radices, threads and every shared index of every pass
+        const InnerPlan& ip = a.ip;
+        if (ip.L != a.n || ip.rmax != 16 || ip.npass < 1 || ip.npass > kRagMaxPass || a.W < 1 || a.threads < 32 ||
+            a.threads % 32 || a.threads > kDTileThreads || a.W * ((int64_t)a.n / 2 + 1) >= (1 << 30) ||
+            a.ntf >= (int64_t(1) << 31) - 64 || a.smem_bytes > kMaxSmemBytes)
+            return fail(why, "dtile plan");
+        if (a.t_fast && (a.W & (a.W - 1))) return fail(why, "dtile columns");
+        auto pad = [&](int i) { return i + (i >> a.pshift); };
+        int64_t ns = 1;
+        for (int p = 0; p < ip.npass; ++p) {
+            const PassDesc& d = ip.pass[p];
+            const int R = d.radix, nbf = a.n / R, nb = R >= kDTileElems ? 1 : kDTileElems / R;
+            if (R < 1 || R > 16 || a.n % R || d.ns != ns || (int64_t)nb * a.threads < (int64_t)a.W * nbf) return fail(why, "dtile pass");
+            for (int j = 0; j < nbf; ++j) {
+                const int q = ns > 1 ? (int)(((uint64_t)(unsigned)j * d.ns_magic) >> 32) : j;
+                if (q != j / ns) return fail(why, "dtile division");
+                const int i0 = (int)(j / ns * ns * R + j % ns), ws = ns == 1 ? 1 : (int)(ns + (ns >> a.pshift));
+                for (int r = 0; r < R; ++r) {
+                    if ((p > 0 || (a.io & DIO_C2R_PRE)) && pad(j) + r * (nbf + (nbf >> a.pshift)) != pad(j + r * nbf))
+                        return fail(why, "dtile read stride");
+                    if ((p + 1 < ip.npass || (a.io & DIO_R2C_POST)) && pad(i0) + r * ws != pad(i0 + r * (int)ns))
+                        return fail(why, "dtile write stride");
+                }
+            }
+            ns *= R;
+        }
+        const int64_t lp = pad(a.n - 1) + 1;
+        if (ns != a.n || (a.t_fast ? a.W * lp : (a.W - 1) * (int64_t)a.pitch + lp) * 16 > a.smem_bytes ||
+            (!a.t_fast && a.pitch < lp))
+            return fail(why, "dtile buffer");
+        if ((a.io & (DIO_R2C_POST | DIO_C2R_PRE)) && (s.post_off < 0 || s.post_off % 2 || s.post_off + 2 * ((int64_t)a.n + 1) > tw_count))
+            return fail(why, "dtile post table");
+    }
     if (a.n < 1 || a.radix < 1 || a.radix > 47 || a.n % a.radix || a.ns < 1 || (a.n / a.radix) % a.ns)
         return fail(why, "dpass radix");
     if (a.ntf < 1 || a.in_split < 1 || a.out_split < 1 || a.in_stride < 1 || a.out_stride < 1)
@@ -358,7 +392,12 @@ bool check_dpass(const Step& s, const Bufs& b, int64_t tw_count, std::string& wh
     const bool herm = (a.io & DIO_HERM_IN) != 0, real_in = (a.io & DIO_REAL_IN) != 0;
     const bool half = (a.io & DIO_HALF_OUT) != 0, real_out = (a.io & DIO_REAL_OUT) != 0;
     int64_t in_last = herm ? a.n / 2 : a.n - 1, out_last = half ? a.n / 2 : a.n - 1;
-    if (a.io & (DIO_R2C_POST | DIO_C2R_PRE)) {
+    if (a.tile && (a.io & (DIO_R2C_POST | DIO_C2R_PRE))) {
+        // rows of n values and of n + 1 bins
+        if (a.in_split != 1 || a.out_split != 1 || a.in_stride != 1 || a.out_stride != 1 || s.src == s.dst)
+            return fail(why, "dtile real layout");
+        ((a.io & DIO_R2C_POST) ? out_last : in_last) = a.n;
+    } else if (a.io & (DIO_R2C_POST | DIO_C2R_PRE)) {
         // the real-data step of an even N = 2L: rows of L values and of L + 1 bins
         if (a.n % 2 || a.radix != 1 || a.ns != 1 || a.in_split != 1 || a.out_split != 1 || a.in_stride != 1 ||
             a.out_stride != 1)
@@ -372,7 +411,9 @@ bool check_dpass(const Step& s, const Bufs& b, int64_t tw_count, std::string& wh
         (max_base(a.out_split, a.out_hi, a.out_lo) + out_last * a.out_stride + 1) * (real_out ? 8 : 16);
     if (in_need > b.bytes[s.src]) return fail(why, "dpass input out of bounds");
     if (out_need > b.bytes[s.dst]) return fail(why, "dpass output out of bounds");
-    if (s.src == s.dst) return fail(why, "dpass in place");
+    const bool alike = a.in_split == a.out_split && a.in_hi == a.out_hi && a.in_lo == a.out_lo &&
+                       a.in_stride == a.out_stride && a.io == 0;
+    if (s.src == s.dst && !(a.tile && alike)) return fail(why, "dpass in place");
     return true;
 }
 

@@ -235,11 +235,11 @@ constexpr int64_t kTileMaxCols = (int64_t(1) << 31) - 64;  // 32-bit column arit
 
 }  // namespace
 
-int tile_threads(int L, const std::vector<int>& rad)
+int tile_threads(int L, const std::vector<int>& rad, int elems)
 {
     int t = 1;
     for (int r : rad) {
-        const int nb = r >= kTileElems ? 1 : kTileElems / r;
+        const int nb = r >= elems ? 1 : elems / r;
         t = std::max(t, (int)ceil_div(L / r, nb));
     }
     return t;
@@ -250,7 +250,7 @@ int tile_threads(int L, const std::vector<int>& rad)
 // addresses of a butterfly an arithmetic sequence, the others descending.
 // c2r: the first pass reads the exchange buffer too (the Hermitian
 // pre-process wrote it), so L/R0 has to be a multiple of a power-of-two R0.
-std::vector<int> choose_tile_radices(int L, bool c2r, int max_threads)
+std::vector<int> choose_tile_radices(int L, bool c2r, int max_threads, int elems)
 {
     if (L == 1) return {1};
     std::vector<int> best, cur;
@@ -258,7 +258,7 @@ std::vector<int> choose_tile_radices(int L, bool c2r, int max_threads)
     std::function<void(int, int)> dfs = [&](int rem, int maxr) {
         if ((int)cur.size() > best_np || (int)cur.size() >= kMaxPass) return;
         if (rem == 1) {
-            const int np = (int)cur.size(), t = tile_threads(L, cur);
+            const int np = (int)cur.size(), t = tile_threads(L, cur, elems);
             if (t > max_threads) return;
             const int mn = *std::min_element(cur.begin(), cur.end());
             if (np < best_np || (np == best_np && (t < best_t || (t == best_t && mn > best_min)))) {
@@ -1101,7 +1101,68 @@ struct DLayout {
     int64_t split = 1, hi = 0, lo = 0, stride = 1;
 };
 
-// Double precision: every axis as global-memory Stockham passes
+// One launch for ntf double-precision transforms of length n (csrc/dtile.cu);
+// false when n needs more than one CTA or a radix above 16.  c2r: with the
+// Hermitian pre-process.
+bool make_dtile(int64_t n, int64_t ntf, bool t_fast, bool c2r, DPassArgs& a)
+{
+    if (n > 8192 || ntf >= kTileMaxCols) return false;
+    const std::vector<int> rad = choose_tile_radices((int)n, c2r, kDTileThreads, kDTileElems);
+    if (rad.empty()) return false;
+    TwiddleBuilder scratch;  // the tables of ip are FP32 and unused
+    const int T = tile_threads((int)n, rad, kDTileElems);
+    if ((int)rad.size() > kRagMaxPass || !build_inner((int)n, rad, T, scratch, a.ip)) return false;
+    const int ps = tile_pshift((int)n, rad, c2r);
+    const int64_t lp = n + (n >> ps);
+    int W = 1, threads = 0;
+    if (t_fast) {
+        // 8 columns (128-byte segments) where the threads allow it
+        W = 8;
+        while (W > 1 && W * T > kDTileThreads) W >>= 1;
+        threads = (W * T + 31) / 32 * 32;
+    } else {
+        // the rows per CTA whose passes fill the lanes of their warps best
+        // (a tie goes to fewer; few transforms keep one row a CTA)
+        double best = 0;
+        for (int w = 1; w * T <= kDTileThreads + 31 && w <= 64 && w * (lp | 1) * 16 <= 72 * 1024; ++w) {
+            int64_t need = 32, cost = 0;
+            for (int r : rad) {
+                const int64_t nb = r >= kDTileElems ? 1 : kDTileElems / r, bf = w * (n / r);
+                need = std::max(need, ceil_div(bf, nb));
+                cost += ceil_div(bf, 32) * r;
+            }
+            need = (need + 31) / 32 * 32;
+            if (need > kDTileThreads) break;
+            const double c = (double)cost / w;
+            if (threads == 0 || c < 0.98 * best) {
+                best = c;
+                W = w;
+                threads = (int)need;
+            }
+            if (ntf / w < 304) break;
+        }
+        if (threads == 0) return false;
+    }
+    const int64_t pitch = t_fast ? 1 : lp | 1;
+    const int64_t smem = (t_fast ? W * lp : W * pitch) * 16;
+    if (smem > kMaxSmemBytes) return false;
+    a.tile = 1;
+    a.n = (int32_t)n;
+    a.radix = 1;
+    a.ns = 1;
+    a.ntf = ntf;
+    a.t_fast = t_fast ? 1 : 0;
+    a.W = W;
+    a.threads = threads;
+    a.pshift = ps;
+    a.pitch = (int32_t)pitch;
+    a.smem_bytes = (int32_t)smem;
+    a.scale = 1.0;
+    return true;
+}
+
+// Double precision: every axis that fits one CTA in one launch
+// (csrc/dtile.cu), the others as global-memory Stockham passes
 // (csrc/dfft.cu).  A pass never writes the buffer it reads: the passes of an
 // axis go src -> WS / WS2 (alternating) -> ... -> OUT, one launch per radix.
 bool build_dsteps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& out, int64_t& ws_bytes,
@@ -1121,11 +1182,38 @@ bool build_dsteps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& 
     // (in_ws: the last pass writes a workspace instead of the output, for a
     // step that follows; `cur` then names that workspace)
     auto axis = [&](int64_t n, int64_t ntf, DLayout src, DLayout mid, DLayout dst, int io_first, int io_last,
-                    bool t_fast, bool in_ws = false) -> bool {
+                    bool t_fast, bool in_ws = false, bool c2r = false) -> bool {
         const std::vector<int> rad = choose_radices((int)n);
         if (rad.empty()) return false;
         const int k = (int)rad.size();
         const int64_t toff = tb.add_dtable(n);
+        {
+            // one launch; in place only where both sides are laid out alike
+            Step st;
+            st.kind = Step::DPASS;
+            const int to = in_ws ? (cur == BUF_WS ? BUF_WS2 : BUF_WS) : BUF_OUT;
+            const DLayout& lo = in_ws ? mid : dst;
+            const bool alike = src.split == lo.split && src.hi == lo.hi && src.lo == lo.lo && src.stride == lo.stride &&
+                               io_first == 0 && io_last == 0;
+            if ((cur != to || alike) && make_dtile(n, ntf, t_fast, c2r, st.dp)) {
+                DPassArgs& a = st.dp;
+                a.io = io_first | io_last;
+                a.in_split = src.split;
+                a.in_hi = src.hi;
+                a.in_lo = src.lo;
+                a.in_stride = src.stride;
+                a.out_split = lo.split;
+                a.out_hi = lo.hi;
+                a.out_lo = lo.lo;
+                a.out_stride = lo.stride;
+                st.dtw_off = toff;
+                st.src = cur;
+                st.dst = to;
+                out.steps.push_back(st);
+                cur = to;
+                return true;
+            }
+        }
         int from = cur;
         int next_ws = (from == BUF_WS) ? BUF_WS2 : BUF_WS;
         int64_t ns = 1;
@@ -1264,7 +1352,25 @@ bool build_dsteps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& 
         a.in_split = a.out_split = 1;
         a.in_stride = a.out_stride = 1;
         pp.dtw_off = toff;
-        if (d2z) {
+        // packing and transform in one launch when it fits and nothing is
+        // overwritten that is still to be read (rows of both sides differ)
+        Step one;
+        one.kind = Step::DPASS;
+        if (src != BUF_OUT && make_dtile(L, rows, false, !d2z, one.dp)) {
+            DPassArgs& f = one.dp;
+            f.io = d2z ? DIO_PAIR_IN | DIO_R2C_POST : DIO_C2R_PRE | DIO_PAIR_OUT;
+            f.in_split = f.out_split = 1;
+            f.in_stride = f.out_stride = 1;
+            f.in_hi = d2z ? L : nb;
+            f.out_hi = d2z ? nb : L;
+            f.conj_out = d2z ? 0 : 1;
+            one.dtw_off = tb.add_dtable(L);
+            one.post_off = toff;
+            one.src = src;
+            one.dst = BUF_OUT;
+            out.steps.push_back(one);
+            cur = BUF_OUT;
+        } else if (d2z) {
             if (!axis(L, rows, rowL, rowL, rowL, DIO_PAIR_IN, 0, false, true))
                 return unsupported("length not decomposable");
             a.io = DIO_R2C_POST;
@@ -1281,7 +1387,7 @@ bool build_dsteps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& 
             pp.dst = src == BUF_WS2 ? BUF_WS : BUF_WS2;
             out.steps.push_back(pp);
             cur = pp.dst;
-            if (!axis(L, rows, rowL, rowL, rowL, 0, DIO_PAIR_OUT, false)) return unsupported("length not decomposable");
+            if (!axis(L, rows, rowL, rowL, rowL, 0, DIO_PAIR_OUT, false, false, true)) return unsupported("length not decomposable");
             out.steps.back().dp.conj_out = 1;  // the backward transform as a forward one
         }
         need(rows * std::max<int64_t>(L, nb) * 16, rows * std::max<int64_t>(L, nb) * 16);

@@ -38,11 +38,12 @@ bool clusters_enabled();
 std::vector<int> choose_radices(int L);
 
 // Tile kernel plans (csrc/tile_fft.cuh): the radices of an on-chip transform
-// of length L, the threads they need at 16 elements each, and the shared
+// of length L, the threads they need at `elems` elements each (a radix above
+// that is one butterfly a thread), and the shared
 // padding shift that goes with them.  c2r: the first pass reads the exchange
 // buffer too (the Hermitian pre-process wrote it).
-std::vector<int> choose_tile_radices(int L, bool c2r = false, int max_threads = 1 << 30);
-int tile_threads(int L, const std::vector<int>& rad);
+std::vector<int> choose_tile_radices(int L, bool c2r = false, int max_threads = 1 << 30, int elems = 16);
+int tile_threads(int L, const std::vector<int>& rad, int elems = 16);
 int tile_pshift(int L, const std::vector<int>& rad, bool c2r = false);
 
 // Split an axis of length n into on-chip factors, each <= cap.

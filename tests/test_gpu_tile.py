@@ -228,3 +228,49 @@ def test_long_real_rows(n, b):
     _ok(ad.cpu().numpy(), n * np.fft.irfft(Xe / w, n), n, ("r2c adjoint", n))
     _ok(bd.cpu().numpy(), np.fft.rfft(x.astype(np.float64)) * w, n, ("c2r adjoint", n))
     _ok(iq[:n * b].cpu().numpy().reshape(b, n), x.astype(np.float64), n * n, ("round trip", n))
+
+
+# double precision: every radix, one and several passes, rows that do not fill
+# a CTA, the longest rows of one launch, columns, even and odd real lengths,
+# in place.  FP64 rounding is 2^-53: the same bound with that unit.
+@pytest.mark.parametrize("n,b", [(r, 7) for r in range(2, 17)] + [(30, 33), (96, 5), (143, 2), (210, 70), (1000, 3), (1500, 2),
+                                                                 (2310, 5), (3375, 1), (4096, 2), (7680, 1), (8192, 1)])
+def test_double_rows(n, b):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((b, n)) + 1j * rng.standard_normal((b, n))
+    r = rng.standard_normal((b, n))
+    X = rng.standard_normal((b, n // 2 + 1)) + 1j * rng.standard_normal((b, n // 2 + 1))
+    st = torch.cuda.current_stream()
+    bound = 4.0 * 2.0 ** -53 * max(math.log2(n), 2.0)  # both sides round
+    with A.Plan.plan1d(n, A.Z2Z, b) as p, A.Plan.plan1d(n, A.D2Z, b) as q, A.Plan.plan1d(n, A.Z2D, b) as s:
+        assert p.check() == "ok" and q.check() == "ok" and s.check() == "ok"
+        for h in (p, q, s):
+            h.set_stream(st)
+        xd, rd, Xd = torch.from_numpy(x).cuda(), torch.from_numpy(r).cuda(), torch.from_numpy(X).cuda()
+        yd, zd, Rd, sd = torch.empty_like(xd), xd.clone(), torch.empty_like(Xd), torch.empty_like(rd)
+        p.exec_z2z(xd, yd, A.FORWARD)
+        p.exec_z2z(zd, zd, A.BACKWARD)
+        q.exec_d2z(rd, Rd)
+        s.exec_z2d(Xd, sd)
+        ip = torch.zeros(2 * (n // 2 + 1) * b, dtype=torch.float64, device="cuda")
+        ip[:n * b] = rd.reshape(-1)
+        q.exec_d2z(ip, ip)
+    for got, want in ((yd, np.fft.fft(x)), (zd, np.fft.ifft(x, norm="forward")), (Rd, np.fft.rfft(r)),
+                      (sd, n * np.fft.irfft(X, n))):
+        e = O.errors(got.cpu().numpy(), want)
+        assert e["rel_l2"] <= bound, (n, b, e)
+    e = O.errors(ip.cpu().numpy().view(np.complex128).reshape(b, -1), np.fft.rfft(r))
+    assert e["rel_l2"] <= bound, (n, b, e)
+
+
+@pytest.mark.parametrize("b,nx,ny", [(2, 33, 10), (1, 512, 7), (3, 60, 64), (1, 2048, 5), (1, 6000, 3)])
+def test_double_columns(b, nx, ny):
+    rng = np.random.default_rng(nx)
+    x = rng.standard_normal((b, nx, ny)) + 1j * rng.standard_normal((b, nx, ny))
+    xd = torch.from_numpy(x).cuda()
+    with A.Plan.plan2d(b, nx, ny, A.Z2Z) as p:
+        assert p.check() == "ok"
+        p.set_stream(torch.cuda.current_stream())
+        p.exec_z2z(xd, xd, A.FORWARD)
+    e = O.errors(xd.cpu().numpy(), np.fft.fft2(x))
+    assert e["rel_l2"] <= 4.0 * 2.0 ** -53 * math.log2(nx * ny), e
