@@ -1,6 +1,9 @@
 // tile_fft.cu - launchers of the tile kernel (instances in tile_io*.cu).
+#include <initializer_list>
+
 #include "launch_common.cuh"
 #include "tile_fft.cuh"
+#include "tile_list.h"
 
 namespace gfft {
 int launch_tile_io0(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
@@ -10,7 +13,25 @@ int launch_tile_io2(const TileArgs& t, int threads, size_t smem, unsigned grid, 
 int launch_tile_io3(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
 int launch_tile_io4(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
 
+#define GFFT_DECL_SHAPE(ID, ...) \
+    int launch_tile_s##ID(int io, const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
+GFFT_TILE_ROWS(GFFT_DECL_SHAPE)
+GFFT_TILE_COLS(GFFT_DECL_SHAPE)
+#undef GFFT_DECL_SHAPE
+
 namespace {
+
+// Whether a launch's tile is the compile-time shape L, T, W, radices.
+bool shape_is(const TileArgs& t, int L, int T, int W, bool rows, std::initializer_list<int> rad)
+{
+    if (t.ip.L != L || t.ip.nthr != T || t.W != W || (t.rows != 0) != rows || t.ip.npass != (int)rad.size()) return false;
+    int p = 0;
+    for (int r : rad)
+        if (t.ip.pass[p++].radix != r) return false;
+    int k = 0;  // the shared padding that goes with them
+    while ((1 << k) < *rad.begin()) ++k;
+    return t.pshift == (rad.size() > 1 && (1 << k) == *rad.begin() ? k : 30);
+}
 
 int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
 {
@@ -21,11 +42,23 @@ int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
     const unsigned per = t.rows || !t.M ? (unsigned)t.W : (unsigned)t.W / 2;  // paired columns: two per unit
     if (per < 1) return (int)cudaErrorInvalidValue;
     const unsigned grid = (t.ncols + per - 1) / per;
+    const bool wide = (int64_t)t.ip.L * (t.in_st8 > t.out_st8 ? t.in_st8 : t.out_st8) > 0xffffffffll;
+    if (!wide && (io == IO_C2C || io == IO_R2C_EVEN || io == IO_C2R_EVEN)) {
+        int rc = kNoTileShape;
+#define GFFT_SHAPE_ROW(ID, LL, TT, WW, ...) \
+    if (shape_is(t, LL, TT, WW, true, {__VA_ARGS__})) rc = launch_tile_s##ID(io, t, threads, smem, grid, st);
+#define GFFT_SHAPE_COL(ID, LL, TT, WW, ...) \
+    if (shape_is(t, LL, TT, WW, false, {__VA_ARGS__})) rc = launch_tile_s##ID(io, t, threads, smem, grid, st);
+        GFFT_TILE_ROWS(GFFT_SHAPE_ROW)
+        GFFT_TILE_COLS(GFFT_SHAPE_COL)
+#undef GFFT_SHAPE_ROW
+#undef GFFT_SHAPE_COL
+        if (rc != kNoTileShape) return rc;
+    }
     switch (io) {
     case IO_C2C:
         // the span of one transform decides the offset width
-        if ((int64_t)t.ip.L * (t.in_st8 > t.out_st8 ? t.in_st8 : t.out_st8) > 0xffffffffll)
-            return launch_tile_io0w(t, threads, smem, grid, st);
+        if (wide) return launch_tile_io0w(t, threads, smem, grid, st);
         return launch_tile_io0(t, threads, smem, grid, st);
     case IO_R2C_EVEN: return launch_tile_io1(t, threads, smem, grid, st);
     case IO_C2R_EVEN: return launch_tile_io2(t, threads, smem, grid, st);
@@ -67,6 +100,8 @@ extern "C" int gfft_launch_tile_row(const RowArgs* a, void* stream)
     t.weight = a->weight;
     t.nreal = a->nreal;
     t.scale = a->scale;
+    t.wl = a->wload;
+    t.wdist = a->wdist;
     return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
 }
 

@@ -1,6 +1,8 @@
 // tile_fft.cuh - on-chip transforms of any length whose radices are at most
 // 16, register to register: the kernel behind every strided ("column") pass
-// and every contiguous row of a length without a compile-time build.
+// and every contiguous row of device memory.  Common lengths are compiled in
+// (TileSpec, tile_list.h), any other runs on the same code with its length,
+// threads and radices as arguments.
 //
 // A CTA takes a TILE of W transforms, T threads each, and a thread holds up
 // to 16 elements.  The first pass loads its butterflies' inputs straight
@@ -84,6 +86,8 @@ struct TileArgs {
     int32_t otw_shift;
     int32_t conj_in, conj_out, weight, nreal;
     float scale;
+    const float* wl;     // even C2R rows: per-bin input weights (row c at c*wdist), or nullptr
+    int64_t wdist;
 };
 
 extern __shared__ __align__(16) float2 tsm[];  // the exchange buffer
@@ -117,15 +121,44 @@ __device__ __forceinline__ void tst(void* base, OFF off, float2 x)
     *reinterpret_cast<float2*>(static_cast<char*>(base) + off) = x;
 }
 
+// Compile-time shape of a tile (csrc/tile_list.h); TileDyn, L = 0, leaves it
+// to the arguments.
+struct TileDyn {
+    static constexpr int L = 0, T = 0, W = 0, NP = 0;
+    static constexpr bool ROWS = false;
+    __host__ __device__ static constexpr int ns(int) { return 0; }
+};
+template <int L_, int T_, int W_, bool ROWS_, int... Rs>
+struct TileSpec {
+    static constexpr int L = L_, T = T_, W = W_, NP = sizeof...(Rs);
+    static constexpr bool ROWS = ROWS_;
+    static constexpr int R[NP] = {Rs...};
+    __host__ __device__ static constexpr int ns(int p)
+    {
+        int n = 1;
+        for (int i = 0; i < p; ++i) n *= R[i];
+        return n;
+    }
+    __host__ __device__ static constexpr int shift()
+    {
+        int k = 0;
+        while ((1 << k) < R[0]) ++k;
+        return NP > 1 && (1 << k) == R[0] ? k : 30;
+    }
+};
+
 // One pass: radix R, up to 16 / R butterflies per thread, all their inputs
 // in registers before any output is written.
-template <int R, int IO, class OFF, bool FIRST, bool LAST>
+template <int R, int IO, class OFF, bool FIRST, bool LAST, class S = TileDyn, int P = 0>
 __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, int p, bool to_global)
 {
     constexpr int NB = R >= 16 ? 1 : 16 / R;
+    constexpr bool ST = S::L > 0;
     const PassDesc& pd = A.ip.pass[p];
     const int nbf = c.L / R;
-    const int ns = pd.ns;
+    const int ns = ST ? S::ns(P) : pd.ns;
+    const bool staged = !(ST && S::ROWS) && A.staged_out;
+    const int64_t in_st8 = ST && S::ROWS ? 8 : A.in_st8, out_st8 = ST && S::ROWS ? 8 : A.out_st8;
     float2 v[NB * R];
     if constexpr (FIRST) {
         if constexpr (IO == IO_R2C_ODD) {
@@ -161,12 +194,12 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
                 }
             });
         } else {
-            const OFF st = (OFF)nbf * (OFF)A.in_st8;
+            const OFF st = (OFF)nbf * (OFF)in_st8;
             sfor<NB>([&](auto bb) {
                 constexpr int b = decltype(bb)::value;
                 const int j = c.tid + b * c.T;
                 if (c.ok && j < nbf) {
-                    const OFF g = (OFF)j * (OFF)A.in_st8;
+                    const OFF g = (OFF)j * (OFF)in_st8;
                     sfor<R>([&](auto rr) {
                         constexpr int r = decltype(rr)::value;
                         v[b * R + r] = tld(c.gi, g + r * st);
@@ -179,7 +212,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
                     v[i].y = -v[i].y;
                 });
             }
-            if (A.otw) {
+            if (!(ST && S::ROWS) && A.otw) {
                 sfor<NB>([&](auto bb) {
                     constexpr int b = decltype(bb)::value;
                     const int j = c.tid + b * c.T;
@@ -193,7 +226,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
                         });
                     }
                 });
-            } else if (A.otw_hi) {
+            } else if (!(ST && S::ROWS) && A.otw_hi) {
                 const unsigned mask = (1u << A.otw_shift) - 1u;
                 sfor<NB>([&](auto bb) {
                     constexpr int b = decltype(bb)::value;
@@ -231,7 +264,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
         if (c.ok && j < nbf) {
             int q = j, k = 0;
             if (ns > 1) {
-                q = fdiv(j, pd);
+                q = ST ? j / ns : fdiv(j, pd);
                 k = j - q * ns;
                 const float2* w = A.tw + pd.tw_off + k;
                 sfor<R - 1>([&](auto rr) {
@@ -242,7 +275,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
             DFT<R>::run(&v[b * R]);
             if (!LAST || !to_global) {
                 int base, ws;
-                if (LAST && A.staged_out) {
+                if (LAST && staged) {
                     base = c.c * A.spitch + j;
                     ws = ns;
                 } else {
@@ -270,8 +303,8 @@ __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, i
                         v[b * R + r].x * A.scale;
                 });
             } else {
-                const OFF g = (OFF)j * (OFF)A.out_st8;
-                const OFF st = (OFF)ns * (OFF)A.out_st8;
+                const OFF g = (OFF)j * (OFF)out_st8;
+                const OFF st = (OFF)ns * (OFF)out_st8;
                 const float2 sc = make_float2(A.scale, A.conj_out ? -A.scale : A.scale);
                 sfor<R>([&](auto rr) {
                     constexpr int r = decltype(rr)::value;
@@ -325,33 +358,49 @@ __device__ __forceinline__ bool tile_pair(const TileArgs& A, uint32_t q, uint32_
     return u != 0 && 2 * u != A.M;
 }
 
+template <class S>
+struct TileShift {
+    static constexpr int value = S::shift();
+};
+
 // OFF: byte offsets within one transform, 32 bits (one add per access) unless
 // its span needs 64 (columns more than 4 GB long).
-template <int MAXT, int MINB, int IO, class OFF = uint32_t>
+template <int MAXT, int MINB, int IO, class OFF = uint32_t, class S = TileDyn>
 __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant__ TileArgs A)
 {
+    constexpr bool ST = S::L > 0;
+    const bool rows = ST ? S::ROWS : A.rows != 0;
     TileCtx c;
-    c.L = A.ip.L;
-    c.T = A.ip.nthr;
-    c.ps = A.pshift;
-    c.em = A.emul;
-    if (A.rows) {
-        c.c = (int)tdiv(threadIdx.x, A.T);
-        c.tid = threadIdx.x - c.c * c.T;
+    if constexpr (ST) {
+        c.L = S::L;
+        c.T = S::T;
+        c.ps = TileShift<S>::value;
+        c.em = S::ROWS ? 1 : S::W;
+        c.c = S::ROWS ? threadIdx.x / S::T : threadIdx.x % S::W;
+        c.tid = S::ROWS ? threadIdx.x % S::T : threadIdx.x / S::W;
     } else {
-        c.c = threadIdx.x & (A.W - 1);
-        c.tid = threadIdx.x >> A.wshift;
+        c.L = A.ip.L;
+        c.T = A.ip.nthr;
+        c.ps = A.pshift;
+        c.em = A.emul;
+        if (rows) {
+            c.c = (int)tdiv(threadIdx.x, A.T);
+            c.tid = threadIdx.x - c.c * c.T;
+        } else {
+            c.c = threadIdx.x & (A.W - 1);
+            c.tid = threadIdx.x >> A.wshift;
+        }
     }
     const uint32_t c0 = blockIdx.x * (uint32_t)A.W;
     const uint32_t col = c0 + (uint32_t)c.c;
     c.ok = c.c < A.W && c.tid < c.T && col < A.ncols;
     constexpr bool kEven = IO == IO_R2C_EVEN || IO == IO_C2R_EVEN;
     uint32_t item = 0, pu = 0, pj = 0;
-    if (kEven && !A.rows) c.ok = tile_pair(A, (uint32_t)c.c, item, pu, pj) && c.tid < c.T;
+    if (kEven && !rows) c.ok = tile_pair(A, (uint32_t)c.c, item, pu, pj) && c.tid < c.T;
     if (!c.ok) c.c = 0;
     const uint32_t cl = c.ok ? col : 0u;
     c.jm = 0;
-    if (A.rows) {
+    if (rows) {
         c.gi = static_cast<const char*>(A.in) + cl * A.in_dist * (IO == IO_R2C_ODD ? 4 : 8);
         c.go = static_cast<char*>(A.out) + cl * A.out_dist * (IO == IO_C2R_ODD ? 4 : 8);
     } else if constexpr (kEven) {
@@ -372,12 +421,12 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
     }
     pdl_wait();  // every access below may touch the caller's buffers
     c.off = c.c * A.cmul;
-    const int np = A.ip.npass;
-    const bool direct = IO != IO_R2C_EVEN && !A.staged_out;  // the last pass stores to HBM
+    const int np = ST ? S::NP : A.ip.npass;
+    const bool direct = IO != IO_R2C_EVEN && ((ST && S::ROWS) || !A.staged_out);  // the last pass stores to HBM
     if constexpr (IO == IO_C2R_EVEN) {
         // Hermitian pre-process into the exchange buffer, every bin loaded
         // once (see codelet_kernel); the passes then all run from it
-        if (!A.rows) {
+        if (!rows) {
             // column u's samples X[u + r*M] and their mirrors X[L - u - r*M]:
             // column M - u, sample Lq-1-r (column 0: its own sample Lq-r;
             // r = 0 pairs DC with Nyquist)
@@ -443,6 +492,7 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             }
         } else if (c.ok) {
             const bool half = A.weight == WEIGHT_LOAD_HALF;
+            const float* wl = A.wl ? A.wl + cl * A.wdist : nullptr;
             constexpr int U = 4;  // pairs in flight
             for (int k0 = c.tid; k0 <= (c.L >> 1); k0 += U * c.T) {
                 float2 xa[U], xb[U], w[U];
@@ -452,6 +502,10 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
                     xa[u] = tld(c.gi, 8u * k);
                     xb[u] = tld(c.gi, 8u * (c.L - k));
                     w[u] = ldg2(A.post + k);
+                    if (wl) {
+                        xa[u] = cscale(xa[u], __ldg(wl + k));
+                        xb[u] = cscale(xb[u], __ldg(wl + (c.L - k)));
+                    }
                 });
                 sfor<U>([&](auto uu) {
                     constexpr int u = decltype(uu)::value;
@@ -476,6 +530,15 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             }
         }
         __syncthreads();
+    }
+    if constexpr (ST) {
+        sfor<S::NP>([&](auto pp) {
+            constexpr int P = decltype(pp)::value;
+            tile_pass<S::R[P], IO, OFF, P == 0 && IO != IO_C2R_EVEN, P == S::NP - 1, S, P>(A, c, P, direct);
+            if (P + 1 < S::NP) __syncthreads();
+        });
+    } else {
+    if (IO == IO_C2R_EVEN) {
         if (np == 1) {
             GFFT_TILE_SWITCH(0, false, true)
         } else {
@@ -497,6 +560,7 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             __syncthreads();
         }
         GFFT_TILE_SWITCH(np - 1, false, true)
+    }
     }
     if (direct) return;
     __syncthreads();
@@ -532,7 +596,7 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
     }
     if constexpr (IO == IO_R2C_EVEN) {
         // even/odd post-process (see codelet_kernel)
-        if (!A.rows) {
+        if (!rows) {
             // bins u + M*kk of column u and their mirrors: column M - u, bin
             // Lq-1-kk (column 0: its own bin Lq-kk; kk = 0 is DC and Nyquist)
             const uint32_t W2 = (uint32_t)A.W >> 1;

@@ -1,0 +1,4 @@
+// tile shape 14 of tile_list.h
+#include "tile_static.cuh"
+
+GFFT_TILE_TU(14)

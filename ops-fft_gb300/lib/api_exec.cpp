@@ -110,6 +110,10 @@ int launch_list(PlanImpl* impl, const StepList& sl, void* in, void* out, cudaStr
         int rc = 0;
         switch (s.kind) {
         case Step::ROW:
+            if (s.has_dev && !host_in) {
+                s.row = s.dev;
+                s.post_off = s.dev_post_off;
+            }
             s.row.tw = tw;
             s.row.post_tw = s.post_off >= 0 ? tw + s.post_off : nullptr;
             s.row.in = src;

@@ -518,7 +518,15 @@ extern "C" ACLFFT_API int aclfftDebugCheckPlan(aclfftHandle plan, char* msg, int
             std::string why;
             bool ok = true;
             if (s.src < 0 || s.src > 3 || s.dst < 0 || s.dst > 3) ok = fail(why, "buffer id");
-            else if (s.kind == Step::ROW) ok = check_row(s, b, impl->tb.count, why);
+            else if (s.kind == Step::ROW) {
+                ok = check_row(s, b, impl->tb.count, why);
+                if (ok && s.has_dev) {
+                    Step d = s;
+                    d.row = s.dev;
+                    d.post_off = s.dev_post_off;
+                    ok = check_row(d, b, impl->tb.count, why);
+                }
+            }
             else if (s.kind == Step::COL) ok = check_col(s, b, impl->tb.count, why);
             else if (s.kind == Step::PACK) ok = check_pack(s, b, impl->tb.count, why);
             else if (s.kind == Step::TC) ok = check_tc(s, b, impl->tb.count, why);

@@ -448,30 +448,22 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
     return true;
 }
 
-// Whether rows of a length with a compile-time build run on the tile kernel.
-// Measured (us, tile / build): C2C 128 x 131072 42.6 / 110, 256 x 65536 41 /
-// 60, 512 x 32768 47 / 57, 1024 x 16384 44 / 48, 2048 x 8192 46 / 49, 4096 x
-// 4096 51 / 56, but 2048 x 2048 16.6 / 15.9, 4096 x 256 7.5 / 7.1, 512 x 2048
-// 7.5 / 6.8; even real lengths 8192 x 2048 36.7 / 46.6, 512 x 32768 28 / 40,
-// 256 x 65536 31 / 65, but 512 x 2048 5.5 / 4.9, 3000 x 4096 28.7 / 27.0.
-// C2C of 128 and 256 points is faster at every size; below 2^21 points (24
-// MB, where pinned host buffers are used in place, which only the builds do)
-// both gain little.  Adjoints of R2C stay: weighted ones need a build.
-bool tile_beats_codelet(int L, int64_t ntf, int io_mode, int weight)
+// Whether rows of a length with a codelet run on the tile kernel when their
+// buffers are in device memory: at every batch, with the length's tile
+// compiled in too (tile_list.h).  Measured (us, tile / codelet): C2C 128 x 8
+// 2.3 / 3.3, 512 x 16 1.9 / 3.0, 1024 x 64 2.2 / 4.2, 2048 x 64 2.5 / 4.1,
+// 4096 x 128 3.6 / 4.4, 1500 x 8192 35.6 / 42.2, 512 x 32768 43 / 56, 4096 x
+// 4096 44 / 55; R2C 1024 x 64 2.4 / 3.5, 3000 x 64 3.2 / 3.9, 3000 x 4096 23.3
+// / 27.7, 8192 x 4096 54 / 86; C2R 1024 x 64 2.7 / 3.4, 3000 x 4096 27.6 /
+// 28.0, 8192 x 4096 61 / 88.  The codelets keep pinned host buffers used in
+// place, tuned plans and 8192 points (C2R 16384: clusters below 1024 rows).
+bool tile_beats_codelet(int L)
 {
     if (std::getenv("OPS_FFT_CODELET_VARIANT")) return false;
     if (t_hints && (t_hints->codelet_variant >= 0 || t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 ||
                     t_hints->codelet_pp >= 0))
         return false;
-    if (weight == WEIGHT_LOAD_HALF) return false;
-    const int64_t points = L * ntf;
-    const bool pow2 = (L & (L - 1)) == 0;
-    switch (io_mode) {
-    case IO_C2C: return pow2 && L <= 4096 && points >= (L <= 256 ? int64_t(1) << 21 : int64_t(1) << 23);
-    case IO_R2C_EVEN:
-    case IO_C2R_EVEN: return pow2 && (L <= 256 || L == 4096) && points >= int64_t(1) << 21;
-    default: return false;
-    }
+    return L <= 4096;
 }
 
 // Rows of any length with radices <= 16 on the tile kernel.
@@ -547,12 +539,16 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     int maxthr = max_threads_for(rmax);
     int nthr = pick_nthr(L, rad, maxthr);
     int codelet = -1;
-    // large batches of these lengths run faster on the tile kernel although a
-    // compile-time build exists
-    if (tile_beats_codelet(L, ntf, io_mode, weight) &&
-        make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st))
+    if (make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) {
+        Step t;
+        if (tile_beats_codelet(L) &&
+            make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, t)) {
+            st.dev = t.row;
+            st.dev_post_off = t.post_off;
+            st.has_dev = true;
+        }
         return true;
-    if (make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
+    }
     if (make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
     const bool even_mode = io_mode == IO_R2C_EVEN || io_mode == IO_C2R_EVEN;
     const bool staged = nthr < 32 && (io_mode == IO_C2C || io_mode == IO_R2C_EVEN);
@@ -895,6 +891,15 @@ bool cluster_for_batch(int64_t n, int64_t batch)
     if (t_hints && t_hints->cluster == 1) return true;
     const char* v = std::getenv("OPS_FFT_CLUSTER_MAXBATCH");
     return batch <= (v ? (int64_t)std::atoll(v) : (int64_t)0);
+}
+
+// Nothing asks for a cluster or for another row kernel.
+bool row_tile_beats_cluster()
+{
+    return clusters_enabled() && codelets_enabled() && !std::getenv("OPS_FFT_CLUSTER_C") &&
+           !std::getenv("OPS_FFT_CLUSTER_MAXBATCH") && !std::getenv("OPS_FFT_CODELET_VARIANT") &&
+           !(t_hints && (t_hints->cluster >= 0 || t_hints->cluster_c > 0 || t_hints->codelet_variant >= 0 ||
+                         t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 || t_hints->codelet_pp >= 0));
 }
 
 // Strided-axis transform as a list of column passes with buffer routing.
@@ -1621,9 +1626,11 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
     const int64_t in_bytes = r2c ? N * p.batch * 4 : nb * p.batch * 8;
     // A single fused kernel reads rows of one pitch and writes rows of
     // another, so an in-place call first copies the input to the workspace.
-    auto single = [&](int io_mode, int L, int64_t in_dist, int64_t out_dist) {
+    auto single = [&](int io_mode, int L, int64_t in_dist, int64_t out_dist, bool tile = false) {
         Step st;
-        if (!make_row_step(L, p.batch, in_dist, out_dist, io_mode, (int)N, p.weight, tb, st)) return false;
+        if (tile ? !make_tile_row_step(L, p.batch, in_dist, out_dist, io_mode, (int)N, p.weight, tb, st)
+                 : !make_row_step(L, p.batch, in_dist, out_dist, io_mode, (int)N, p.weight, tb, st))
+            return false;
         int src = IN;
         if (inplace) {
             Step cp;
@@ -1644,6 +1651,13 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         const int64_t L = N / 2;
         const int mode = r2c ? IO_R2C_EVEN : IO_C2R_EVEN;
         const bool row_ok = L <= row_max_length() && row_feasible((int)L, mode);
+        // 8192 points also fit one CTA: rows from the batches where its waves
+        // fill the chip, clusters below (us, rows / clusters: R2C 16384 x 64
+        // 6.8 / 7.3, 128 8.2 / 11.4, 4096 129 / 183; C2R 64 7.3 / 6.3, 512
+        // 24.3 / 22.5, 1024 40.9 / 41.5, 4096 144 / 152)
+        if (row_ok && L == 8192 && p.batch >= (r2c ? 64 : 1024) && row_tile_beats_cluster()) {
+            if (single(mode, (int)L, r2c ? L : nb, r2c ? nb : L, true)) return true;
+        }
         if (row_ok && !cluster_for_batch(L, p.batch)) {
             if (!single(mode, (int)L, r2c ? L : nb, r2c ? nb : L)) return false;
             return true;

@@ -55,6 +55,9 @@ struct Step {
     enum Kind { ROW, COL, PACK, COPY, TC, CLUSTER, DPASS } kind = ROW;
     int64_t copy_bytes = 0;
     RowArgs row{};
+    RowArgs dev{};  // ROW with has_dev: the launch for device buffers, `row` the one for mapped host memory
+    bool has_dev = false;
+    int64_t dev_post_off = -1;
     ColArgs col{};
     PackArgs pack{};
     TcArgs tc{};
