@@ -127,6 +127,7 @@ struct TileDyn {
     static constexpr int L = 0, T = 0, W = 0, NP = 0;
     static constexpr bool ROWS = false;
     __host__ __device__ static constexpr int ns(int) { return 0; }
+    __host__ __device__ static constexpr int nb(int R) { return R >= 16 ? 1 : 16 / R; }
 };
 template <int L_, int T_, int W_, bool ROWS_, int... Rs>
 struct TileSpec {
@@ -139,6 +140,7 @@ struct TileSpec {
         for (int i = 0; i < p; ++i) n *= R[i];
         return n;
     }
+    __host__ __device__ static constexpr int nb(int R) { return (L / R + T - 1) / T; }  // butterflies a thread
     __host__ __device__ static constexpr int shift()
     {
         int k = 0;
@@ -152,7 +154,7 @@ struct TileSpec {
 template <int R, int IO, class OFF, bool FIRST, bool LAST, class S = TileDyn, int P = 0>
 __device__ __forceinline__ void tile_pass(const TileArgs& A, const TileCtx& c, int p, bool to_global)
 {
-    constexpr int NB = R >= 16 ? 1 : 16 / R;
+    constexpr int NB = S::nb(R);
     constexpr bool ST = S::L > 0;
     const PassDesc& pd = A.ip.pass[p];
     const int nbf = c.L / R;

@@ -1597,6 +1597,18 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
             if (spare) need_ws(N * p.stride * 8);
             return true;
         }
+        // 8192 points also fit one CTA: from 64 rows faster than a cluster of
+        // four (us: 16 rows 5.5 / 4.7, 64 5.5 / 6.0, 128 7.2 / 8.7, 512 18.9 /
+        // 19.1, 8192 208 / 237)
+        if (N == 8192 && p.batch >= 64 && row_tile_beats_cluster()) {
+            Step st;
+            if (make_tile_row_step((int)N, p.batch, N, N, IO_C2C, 0, WEIGHT_NONE, tb, st)) {
+                st.src = IN;
+                st.dst = BUF_OUT;
+                out.steps.push_back(st);
+                return true;
+            }
+        }
         if (cluster_for_batch(N, p.batch)) {
             Step st;
             if (make_cluster_step(N, p.batch, tb, st)) {
@@ -1661,6 +1673,19 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         if (row_ok && !cluster_for_batch(L, p.batch)) {
             if (!single(mode, (int)L, r2c ? L : nb, r2c ? nb : L)) return false;
             return true;
+        }
+        // two passes over HBM beat a 16-CTA cluster from 8 rows (us, 131072:
+        // R2C x 1 8.9 / 8.6, x 8 10.4 / 11.7, x 64 33 / 46, x 512 223 / 316;
+        // C2R x 512 242 / 323); 65536: R2C 114 / 118, C2R 125 / 123.  Out of
+        // place the middle result sits in the output, in place in the
+        // workspace that the cluster's copy needs too.
+        if (L == 65536 && p.batch >= 8 && row_tile_beats_cluster()) {
+            const std::vector<int> fac = split_axis(L, cap);
+            if (fac.size() == 2 && make_pair_steps(L, p.batch, r2c, p.weight, IN, inplace ? BUF_WS : BUF_OUT,
+                                                   r2c && !inplace ? nb : L, BUF_OUT, fac, tb, out.steps)) {
+                if (inplace) need_ws(L * p.batch * 8);
+                return true;
+            }
         }
         // long real transforms (and short ones in small batches) on a
         // cluster, packing fused (an in-place call first copies the input to

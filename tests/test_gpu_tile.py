@@ -156,7 +156,7 @@ def test_ragged_tiles(lens, kind):
 
 # lengths with a codelet, whose rows in device memory run on the tile kernel
 @pytest.mark.parametrize("n,b", [(128, 16383), (128, 16384), (256, 8192), (512, 16384), (1024, 8192), (2048, 4096),
-                                 (4096, 2048)])
+                                 (4096, 2048), (8192, 63), (8192, 64)])
 def test_rows_of_built_lengths(n, b):
     g = torch.Generator(device="cuda")
     g.manual_seed(n)
@@ -259,10 +259,12 @@ def test_compiled_long_tiles(n, b):
 
 
 # real rows of 16384: clusters below 64 (R2C) and 1024 (C2R) rows, rows in one
-# CTA from there; in place, and no weighted adjoint on either
-@pytest.mark.parametrize("b", [63, 64, 1023, 1024])
-def test_real_rows_16384(b):
-    n, nb = 16384, 8193
+# CTA from there; of 131072: clusters below 8 rows, two passes from there; in
+# place, and no weighted adjoint on any
+@pytest.mark.parametrize("n,b", [(16384, 63), (16384, 64), (16384, 1023), (16384, 1024), (131072, 7), (131072, 8),
+                                 (131072, 33)])
+def test_real_rows_beside_clusters(n, b):
+    nb, least = n // 2 + 1, (64, 1024) if n == 16384 else (8, 8)
     g = torch.Generator(device="cuda")
     g.manual_seed(b)
     x = torch.randn((b, n), generator=g, device="cuda")
@@ -273,7 +275,7 @@ def test_real_rows_16384(b):
         for q in (r, c):
             assert q.check() == "ok"
             q.set_stream(torch.cuda.current_stream())
-        assert (r.info().cluster_ctas > 0) == (b < 64) and (c.info().cluster_ctas > 0) == (b < 1024)
+        assert (r.info().cluster_ctas > 0) == (b < least[0]) and (c.info().cluster_ctas > 0) == (b < least[1])
         r.exec_r2c(x, X)
         c.exec_c2r(X, y)
         r.exec_r2c_adjoint(X, gd)
