@@ -1,6 +1,6 @@
 // codelet_inst.cuh - one translation unit per codelet_list.h entry:
 // a codelet_<id>.cu file holds GFFT_CODELET_TU(<id>), which instantiates
-// that entry's row and column-tile kernels and their launchers only.
+// that entry's row kernels and their launchers only.
 #pragma once
 #include "codelet.cuh"
 #include "codelet_list.h"

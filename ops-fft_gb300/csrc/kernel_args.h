@@ -247,14 +247,23 @@ struct RagRow {
     int64_t in_off, out_off;
 };
 
+enum RagClaim : int {
+    RAG_CLAIM_NONE = 0,  // CTA b runs item b (at most one item a CTA, no dependencies); the queue is not used
+    RAG_CLAIM_NEXT = 1,  // the next item when one is done
+    RAG_CLAIM_AHEAD = 2  // two items ahead
+};
+
 struct RagArgs {
     const RagItem* items;
     const RagRow* rows;
     int32_t nitems;
     int32_t smem_bytes;
     int32_t ctas;   // persistent CTAs to launch (gfft_ragged_ctas * SM count)
+    int32_t claim;      // RagClaim
     int32_t need_bias;  // added to every dependency count (test hook; 0 normally)
-    int* queue;     // queue[0]: next item; queue[1 + x]: completed items of transform x
+    int32_t count;  // transforms
+    int* queue;     // queue[0]: next item; queue[1 + x]: completed items of transform x; queue[1 + count]: CTAs done.
+                    // All zero before a launch, and again after it
     int* err;
     const void* tw;
     const void* in;

@@ -1,7 +1,6 @@
 // ragged.cu - ragged batches of transforms in one persistent launch.
 //
-// Every CTA (256 threads, four per SM; 512 for a batch with a length that
-// needs them) loops over work items claimed from the
+// Every CTA (512 threads, two per SM) loops over work items claimed from the
 // queue head.  An item is a tile of the register-to-register scheme of
 // tile_fft.cuh with its lengths, strides, radices and table offsets in a
 // 240-byte record:
@@ -16,17 +15,21 @@
 //               `count` neighbouring elements a row;
 //   RAG_POST    a range of the even/odd post-process of a long even R2C.
 //
-// The index after the next one is claimed (one atomic) and the next record
-// copied (cp.async) while an item is processed; a finished item is published
+// With eight items or more a CTA the index after the next one is claimed (one
+// atomic) and the next record copied (cp.async) while an item is processed; a finished item is published
 // after the next item's first barrier, when its stores have drained.  Claims
 // ahead cannot deadlock: a CTA's claims increase, and every wait is on lower
 // items, so the lowest unfinished item is always being processed.  Waits (P2
-// on P1, POST on P2) are done by one thread with a clock bound.
+// on P1, POST on P2) are done by one thread with a clock bound.  Shorter
+// queues are claimed item by item (a CTA that started early took two items
+// and left others without: 163 transforms of up to 8192 points 26 -> 21 us),
+// and when every item has a CTA and none waits, CTA b takes item b.
 //
 // What bounds it: issue and latency at 32 warps per SM (issue 30 % active,
 // warps waiting on loads 5.9, at barriers 4.6 per issue).  10000 transforms
-// of 16..32768 points: 977 -> 512 us against the staged shared-memory passes
-// this replaced.  Measured and left out: CTAs of 256 threads, four per SM
+// of 16..32768 points: 977 -> 419 us against the staged shared-memory passes
+// this replaced; 163 of up to 8192, one or two items a CTA with cold code,
+// 17.2 -> 19.9.  Measured and left out: CTAs of 256 threads, four per SM
 // (one length 10 % faster, mixed lengths 516 us); HBM reads started one round
 // of the grid ahead with bulk L2 prefetches (515 us); one copy of each radix'
 // code for first, inner and last passes (559 us).
@@ -276,8 +279,8 @@ __global__ void __launch_bounds__(NT, 2) ragged_kernel(const __grid_constant__ R
     __shared__ int s_ok;
     const int t = threadIdx.x;
     if (t == 0) {
-        s_claim[0] = atomicAdd(A.queue, 1);
-        s_claim[1] = atomicAdd(A.queue, 1);
+        s_claim[0] = A.claim == RAG_CLAIM_NONE ? (int)blockIdx.x : atomicAdd(A.queue, 1);
+        s_claim[1] = A.claim == RAG_CLAIM_AHEAD ? atomicAdd(A.queue, 1) : A.nitems;
     }
     __syncthreads();
     int it = s_claim[0], nxt = s_claim[1];
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(NT, 2) ragged_kernel(const __grid_constant__ R
     for (int cur = 0; it < A.nitems; cur ^= 1) {
         // run ahead: claim the item after the next one, fetch the next record
         int claimed = 0;
-        if (t == NT - 1) claimed = atomicAdd(A.queue, 1);
+        if (t == NT - 1) claimed = A.claim == RAG_CLAIM_AHEAD ? atomicAdd(A.queue, 1) : A.nitems;
         if (t < kRecChunks && nxt < A.nitems)
             cp_async16(reinterpret_cast<unsigned char*>(&s_rec[cur ^ 1]) + 16 * t,
                        reinterpret_cast<const unsigned char*>(A.items + nxt) + 16 * t);
@@ -406,11 +409,34 @@ __global__ void __launch_bounds__(NT, 2) ragged_kernel(const __grid_constant__ R
         __syncthreads();
         it = nxt;
         nxt = s_claim[cur];
+        if (A.claim == RAG_CLAIM_NONE) return;
+        if (A.claim == RAG_CLAIM_NEXT) {
+            publish();
+            if (t == 0) s_claim[0] = atomicAdd(A.queue, 1);
+            __syncthreads();
+            it = s_claim[0];
+            nxt = A.nitems;
+            if (it < A.nitems && t < kRecChunks)
+                reinterpret_cast<int4*>(&s_rec[cur ^ 1])[t] = __ldg(reinterpret_cast<const int4*>(A.items + it) + t);
+            __syncthreads();
+        }
     }
     if (t == 0 && pending >= 0) {
         __threadfence();
         atomicAdd(A.queue + 1 + pending, 1);
     }
+    if (A.claim == RAG_CLAIM_NONE) return;
+    // the last CTA clears the queue, instead of a memset ahead of every launch
+    // (10000 transforms 438 -> 419 us); no CTA touches it after counting itself
+    __syncthreads();
+    if (t == 0) {
+        __threadfence();
+        s_ok = atomicAdd(A.queue + 1 + A.count, 1) == (int)gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_ok)
+        for (int i = t; i < A.count + 2; i += NT) A.queue[i] = 0;
 }
 
 }  // namespace

@@ -154,6 +154,35 @@ def test_ragged_tiles(lens, kind):
             _ok(y, np.fft.rfft(hin[i:i + n].astype(np.float64)), n, ("ragged r2c", n))
 
 
+# the three ways items are claimed (none: at most one a CTA and no long
+# transform; one by one; ahead), launched again on the queue the last left
+@pytest.mark.parametrize("count,hi", [(40, 4096), (200, 16384), (3000, 32768)])
+def test_ragged_claims(count, hi):
+    lens, kinds = A.ragged_lengths(count, 16, hi, 0.7, 7)
+    ino, outo, ci, co = A.ragged_layout(lens, kinds)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(count)
+    x = torch.randn(ci // 4, generator=g, device="cuda")
+    ys = [torch.zeros(co // 4, device="cuda") for _ in range(3)]
+    with A.RaggedPlan(lens, kinds, ino, outo) as p:
+        p.set_stream(torch.cuda.current_stream())
+        p.set_options(autotune=False, graph=False)
+        assert p.check() == "ok"
+        for y in ys:
+            p.exec(x, y, A.FORWARD)
+        assert p.error_flags() == 0
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+    h, o = x.cpu().numpy(), ys[0].cpu().numpy()
+    for k in list(range(0, count, max(1, count // 60))) + [int(np.argmax(lens))]:
+        n, a, b = int(lens[k]), int(ino[k]) // 4, int(outo[k]) // 4
+        if int(kinds[k]) == int(A.C2C):
+            want = np.fft.fft(h[a:a + 2 * n].view(np.complex64).astype(np.complex128))
+            _ok(o[b:b + 2 * n].view(np.complex64), want, n, (count, k, n))
+        else:
+            want = np.fft.rfft(h[a:a + n].astype(np.float64))
+            _ok(o[b:b + 2 * (n // 2 + 1)].view(np.complex64), want, n, (count, k, n))
+
+
 # lengths with a codelet, whose rows in device memory run on the tile kernel
 @pytest.mark.parametrize("n,b", [(128, 16383), (128, 16384), (256, 8192), (512, 16384), (1024, 8192), (2048, 4096),
                                  (4096, 2048), (8192, 63), (8192, 64)])
