@@ -54,12 +54,12 @@ FALLBACK_HBM_GBS = 6800.0
 # Writes of a launch mostly stay in L2 when the kernel ends, so this is below
 # the algorithmic read+write bytes.
 NCU_TRAFFIC = {
-    ("cfg2", "dominant"): 53330432,  # R2C N=3000 batch=4096: 49.22 MB read + 4.11 MB written
-    ("cfg1", "dominant"): 8472064,   # C2C 4096 x 256 (row codelet): 8.47 MB read, the 8.4 MB output left in L2
+    ("cfg2", "dominant"): 53416704,  # R2C N=3000 batch=4096: 49.19 MB read + 4.23 MB written
+    ("cfg1", "dominant"): 8433920,   # C2C 4096 x 256: 8.43 MB read, the 8.4 MB output left in L2
     ("cfg3", "dominant"): 68792064,  # TF32x3 N=65536 x 64, both passes: 67.19 MB read + 1.60 MB written
-    ("cfg4", "dominant"): 970750000,  # 2D forward: row pass 268.5 + 214.7 MB, column-tile pass 268.5 + 219.0 MB
+    ("cfg4", "dominant"): 964478976,  # 2D forward: row pass 268.5 + 214.7 MB, column pass 268.5 + 212.8 MB
     ("long", "dominant"): 487250944,  # C2C 65536 x 512 on 16-CTA clusters: 268.73 MB read + 218.52 MB written
-    ("cfg5", "dominant"): 1086378752,  # ragged launch: 567.78 MB read + 518.60 MB written (workspace round trip)
+    ("cfg5", "dominant"): 1130139648,  # ragged launch: 560.55 MB read + 569.59 MB written (workspace round trip)
 }
 
 
@@ -397,7 +397,7 @@ class OneExecWorkload:
     """One forward exec per step of a plan beyond the benchmark configurations, for
     measurement and profiling: ``c2c3d`` a 3D C2C of 512^3 (z rows, then
     512-point column tiles along y and x); ``fp64`` a double-precision Z2Z of
-    4096 x 2048 (three FP64 Stockham passes)."""
+    4096 x 2048 (one launch)."""
 
     def __init__(self, torch, A, dev, stream, nsets, kind):
         self.torch, self.A, self.kind = torch, A, kind

@@ -31,8 +31,11 @@
 // registers): 256 x 263168 columns 232 -> 168 us (0.945), 2310 x 4096 rows
 // 53.1 -> 37.5 us (0.594); at 48 registers, with spills, 195 and 36.2 us.
 // Against the kernels these sizes used before: 387 and 74 us; 512^3 3D
-// 1823 -> 1342 us.  Three radices cost 45 instructions an element, a third
-// of them addresses, and run at 0.6-0.88; two radices at 0.85-0.97.
+// 1823 -> 1342 us.  With lengths as arguments two radices cost 46
+// instructions a point, three 64, a third of them addresses; compiled in, a
+// quarter fewer: 512^3 1033 us (0.92 of the copy rate over its three passes),
+// 4096 x 4096 rows 44 us (0.90), 3000 x 4096 R2C 23.2 us (0.63: odd radices,
+// the post-process; shared-memory pipe 69 %, issue 40 %).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
