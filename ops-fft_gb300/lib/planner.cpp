@@ -657,7 +657,7 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     if (a.ncols >= kTileMaxCols || t_no_tiles) return false;
     const std::vector<int> rad = choose_tile_radices(Lq);
     if (rad.empty()) return false;
-    const int T = tile_threads(Lq, rad);
+    int T = tile_threads(Lq, rad);
     // strided axes: 16 columns (128-byte row segments) where the threads
     // allow it (512-point axes of 512^3: 1283 us against 1489 at 8 columns;
     // 256 x 263168: 169 against 313); passes of a long row, whose segments
@@ -668,6 +668,12 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     if (T * W > kTileMaxThreads) return false;
     // few columns: narrower tiles until two CTAs per SM are there
     while (W > 4 && a.ncols / W < 304) W >>= 1;
+    // and, as for rows, a thread for every butterfly while that leaves at most
+    // 256 threads on an SM (us, without / with: 32 x 30 2D 7.1 / 5.3, 32 x 30 x
+    // 40 12.3 / 9.9, one row of 262144 9.9 / 8.6)
+    int T1 = 1;
+    for (int r : rad) T1 = std::max(T1, Lq / r);
+    if (T1 * W <= kTileMaxThreads && a.ncols * T1 <= 152 * 256) T = T1;
     TwiddleBuilder trial = tb;
     InnerPlan ip;
     if (!build_inner(Lq, rad, T, trial, ip)) return false;

@@ -255,7 +255,7 @@ def test_compiled_row_tiles(L):
 # columns of the compiled lengths and tile widths, as strided axes and as the
 # passes of long rows (staged, with outer twiddles, paired real columns)
 @pytest.mark.parametrize("nx,ny,b", [(128, 125, 40), (256, 72, 70), (256, 9, 2), (512, 80, 64), (512, 24, 128),
-                                     (1024, 40, 64), (2048, 24, 64)])
+                                     (1024, 40, 64), (2048, 24, 64), (32, 30, 1), (512, 60, 1), (1024, 37, 1), (30, 1, 3)])
 def test_compiled_column_tiles(nx, ny, b):
     rng = np.random.default_rng(nx)
     x = (rng.standard_normal((b, nx, ny)) + 1j * rng.standard_normal((b, nx, ny))).astype(np.complex64)
