@@ -35,6 +35,8 @@
 // code for first, inner and last passes (559 us).
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "butterfly.cuh"
 #include "kernel_args.h"
 #include "pipe_ptx.cuh"
@@ -447,9 +449,21 @@ using namespace gfft;
 extern "C" int gfft_ragged_ctas(int smem_bytes)
 {
     // the kernel's static shared memory counts against the opt-in limit, so
-    // the attribute is the dynamic size actually launched with
-    int occ = 0;
-    cudaError_t e = cudaFuncSetAttribute(ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    // the attribute is a dynamic size actually launched with: the largest of
+    // any plan on the device so far, since plans that asked for more are still
+    // launched
+    static std::mutex mu;
+    static int limit[64] = {0};
+    int occ = 0, dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(mu);
+        int& most = limit[dev & 63];
+        if (smem_bytes > most) {
+            e = cudaFuncSetAttribute(ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+            if (e == cudaSuccess) most = smem_bytes;
+        }
+    }
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ragged_kernel, NT, (size_t)smem_bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
