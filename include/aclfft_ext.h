@@ -97,10 +97,11 @@ typedef struct aclfftPlanInfo_t {
     int transforms_per_cta;
     long long twiddle_entries; /* complex entries generated on the GPU */
     size_t workspace_bytes;    /* device workspace owned by the plan */
-    int kernel;                /* first step: -1 tile or generic row/column kernel, >= 0 specialised codelet id (its fields
-                                * below describe the codelet, which pinned host buffers and tuned plans use; device
-                                * buffers may run on the tile kernel) */
-    int groups_per_cta;        /* codelets: independent transform groups per CTA */
+    int kernel;                /* first step: >= 0 the length's specialised codelet, -1 none.  Pinned host buffers and
+                                * tuned plans run on it; device buffers do when groups_per_cta >= 1 */
+    int groups_per_cta;        /* transform groups per CTA of a codelet that device buffers run on; 0: they run on a
+                                * tile or a generic kernel, which the radices, threads, transforms, stages and shared
+                                * memory here then describe */
     int stages;                /* input prefetch stages */
     int smem_bytes;            /* dynamic shared memory per CTA */
     int tc_stages;             /* tensor-core DFT-matrix launches per exec (0: FP32 kernels only) */

@@ -183,12 +183,14 @@ ACLFFT_API aclfftResult aclfftGetPlanInfo(aclfftHandle plan, aclfftPlanInfo* inf
         int tf = 0;
         info->kernel = -1;
         if (s.kind == gfft::Step::ROW) {
-            ip = &s.row.ip;
-            tf = s.row.tfpc;
+            // the launch that device buffers take
+            const gfft::RowArgs& r = s.has_dev ? s.dev : s.row;
+            ip = &r.ip;
+            tf = r.tfpc;
             info->kernel = s.row.codelet;
-            info->groups_per_cta = s.row.ngroups;
-            info->stages = s.row.nstage;
-            info->smem_bytes = s.row.smem_bytes;
+            info->groups_per_cta = r.ngroups;
+            info->stages = r.nstage;
+            info->smem_bytes = r.smem_bytes;
         } else if (s.kind == gfft::Step::COL) {
             ip = &s.col.ip;
             tf = s.col.tfpc;
