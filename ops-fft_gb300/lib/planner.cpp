@@ -448,6 +448,17 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
     return true;
 }
 
+// A switch or a tuned choice that describes a codelet asks for that codelet.
+bool codelet_asked(int io_mode)
+{
+    for (const char* name : {"OPS_FFT_CODELET_VARIANT", "OPS_FFT_CODELET_NG", "OPS_FFT_CODELET_NST", "OPS_FFT_CODELET_PP"})
+        if (std::getenv(name)) return true;
+    const char* fuse = std::getenv("OPS_FFT_FUSE_R2C");
+    if (fuse && fuse[0] == '0' && io_mode == IO_R2C_EVEN) return true;
+    return t_hints && (t_hints->codelet_variant >= 0 || t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 ||
+                       t_hints->codelet_pp >= 0);
+}
+
 // Whether rows of a length with a codelet run on the tile kernel when their
 // buffers are in device memory: at every batch, with the length's tile
 // compiled in too (tile_list.h).  Measured (us, tile / codelet): C2C 128 x 8
@@ -457,14 +468,7 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
 // / 27.7, 8192 x 4096 54 / 86; C2R 1024 x 64 2.7 / 3.4, 3000 x 4096 27.6 /
 // 28.0, 8192 x 4096 61 / 88.  The codelets keep pinned host buffers used in
 // place, tuned plans and 8192 points (C2R 16384: clusters below 1024 rows).
-bool tile_beats_codelet(int L)
-{
-    if (std::getenv("OPS_FFT_CODELET_VARIANT")) return false;
-    if (t_hints && (t_hints->codelet_variant >= 0 || t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 ||
-                    t_hints->codelet_pp >= 0))
-        return false;
-    return L <= 4096;
-}
+bool tile_beats_codelet(int L, int io_mode) { return L <= 4096 && !codelet_asked(io_mode); }
 
 // Rows of any length with radices <= 16 on the tile kernel.
 bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io_mode, int nreal, int weight,
@@ -541,7 +545,7 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     int codelet = -1;
     if (make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) {
         Step t;
-        if (tile_beats_codelet(L) &&
+        if (tile_beats_codelet(L, io_mode) &&
             make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, t)) {
             st.dev = t.row;
             st.dev_post_off = t.post_off;
@@ -549,7 +553,8 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
         }
         return true;
     }
-    if (make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
+    // OPS_FFT_CODELETS=0, or a tuned choice of no codelets, asks for the kernel below
+    if (codelets_enabled() && make_tile_row_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st)) return true;
     const bool even_mode = io_mode == IO_R2C_EVEN || io_mode == IO_C2R_EVEN;
     const bool staged = nthr < 32 && (io_mode == IO_C2C || io_mode == IO_R2C_EVEN);
     const int start = io_mode == IO_C2R_EVEN ? 1 : 0;
@@ -900,12 +905,10 @@ bool cluster_for_batch(int64_t n, int64_t batch)
 }
 
 // Nothing asks for a cluster or for another row kernel.
-bool row_tile_beats_cluster()
+bool row_tile_beats_cluster(int io_mode)
 {
-    return clusters_enabled() && codelets_enabled() && !std::getenv("OPS_FFT_CLUSTER_C") &&
-           !std::getenv("OPS_FFT_CLUSTER_MAXBATCH") && !std::getenv("OPS_FFT_CODELET_VARIANT") &&
-           !(t_hints && (t_hints->cluster >= 0 || t_hints->cluster_c > 0 || t_hints->codelet_variant >= 0 ||
-                         t_hints->codelet_ng > 0 || t_hints->codelet_nst > 0 || t_hints->codelet_pp >= 0));
+    return clusters_enabled() && codelets_enabled() && !codelet_asked(io_mode) && !std::getenv("OPS_FFT_CLUSTER_C") &&
+           !std::getenv("OPS_FFT_CLUSTER_MAXBATCH") && !(t_hints && (t_hints->cluster >= 0 || t_hints->cluster_c > 0));
 }
 
 // Strided-axis transform as a list of column passes with buffer routing.
@@ -1606,7 +1609,7 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         // 8192 points also fit one CTA: from 64 rows faster than a cluster of
         // four (us: 16 rows 5.5 / 4.7, 64 5.5 / 6.0, 128 7.2 / 8.7, 512 18.9 /
         // 19.1, 8192 208 / 237)
-        if (N == 8192 && p.batch >= 64 && row_tile_beats_cluster()) {
+        if (N == 8192 && p.batch >= 64 && row_tile_beats_cluster(IO_C2C)) {
             Step st;
             if (make_tile_row_step((int)N, p.batch, N, N, IO_C2C, 0, WEIGHT_NONE, tb, st)) {
                 st.src = IN;
@@ -1673,7 +1676,7 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         // fill the chip, clusters below (us, rows / clusters: R2C 16384 x 64
         // 6.8 / 7.3, 128 8.2 / 11.4, 4096 129 / 183; C2R 64 7.3 / 6.3, 512
         // 24.3 / 22.5, 1024 40.9 / 41.5, 4096 144 / 152)
-        if (row_ok && L == 8192 && p.batch >= (r2c ? 64 : 1024) && row_tile_beats_cluster()) {
+        if (row_ok && L == 8192 && p.batch >= (r2c ? 64 : 1024) && row_tile_beats_cluster(mode)) {
             if (single(mode, (int)L, r2c ? L : nb, r2c ? nb : L, true)) return true;
         }
         if (row_ok && !cluster_for_batch(L, p.batch)) {
@@ -1685,7 +1688,7 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         // C2R x 512 242 / 323); 65536: R2C 114 / 118, C2R 125 / 123.  Out of
         // place the middle result sits in the output, in place in the
         // workspace that the cluster's copy needs too.
-        if (L == 65536 && p.batch >= 8 && row_tile_beats_cluster()) {
+        if (L == 65536 && p.batch >= 8 && row_tile_beats_cluster(mode)) {
             const std::vector<int> fac = split_axis(L, cap);
             if (fac.size() == 2 && make_pair_steps(L, p.batch, r2c, p.weight, IN, inplace ? BUF_WS : BUF_OUT,
                                                    r2c && !inplace ? nb : L, BUF_OUT, fac, tb, out.steps)) {

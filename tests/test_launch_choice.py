@@ -1,10 +1,17 @@
 """Which launch a plan makes, as aclfftGetPlanInfo reports it: lengths with a
 specialised codelet run on compiled tiles in device memory unless a switch or
 a tuned choice asks for the codelet."""
+import json
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
 import aclfft as A
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _info(n, typ=A.C2C, b=4096):
@@ -26,3 +33,37 @@ def test_info_describes_the_launch_of_device_buffers(n, typ, rad, threads, rows)
     assert i.threads_per_transform == threads and i.transforms_per_cta == rows
     # at most one element of padding in eight, and two to a row
     assert rows * L * 8 <= i.smem_bytes <= rows * (L + L // 8 + 2) * 8
+
+
+@pytest.mark.parametrize("name,value,field,want", [
+    ("OPS_FFT_CODELET_VARIANT", "0", "groups_per_cta", None), ("OPS_FFT_CODELET_NG", "2", "groups_per_cta", 2),
+    ("OPS_FFT_CODELET_NST", "3", "stages", 3), ("OPS_FFT_CODELET_PP", "1", "groups_per_cta", None),
+    ("OPS_FFT_FUSE_R2C", "0", "groups_per_cta", None)])
+def test_codelet_switches_act_on_device_buffers(name, value, field, want, monkeypatch):
+    monkeypatch.setenv(name, value)
+    i = _info(2048, A.R2C)
+    assert i.kernel >= 0 and i.groups_per_cta >= 1
+    assert want is None or getattr(i, field) == want
+
+
+_NO_CODELETS = r"""
+import json, sys
+sys.path[:0] = [sys.argv[1] + "/ops-fft_gb300"]
+import aclfft as A
+out = []
+for n in (4096, 2310):
+    with A.Plan.plan1d(n, A.C2C, 4096) as p:
+        i = p.info()
+        out.append([p.check(), i.kernel, i.groups_per_cta, i.smem_bytes, i.transforms_per_cta * i.onchip_length * 8])
+print(json.dumps(out))
+"""
+
+
+def test_no_codelets_means_the_generic_row_kernel():
+    """OPS_FFT_CODELETS=0 (read once per process): prefetch slots and ping-pong
+    buffers in shared memory, at least twice a tile's one exchange buffer."""
+    env = dict(os.environ, OPS_FFT_CODELETS="0")
+    r = subprocess.run([sys.executable, "-c", _NO_CODELETS, ROOT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    for check, kernel, groups, smem, rows in json.loads(r.stdout.strip().splitlines()[-1]):
+        assert check == "ok" and kernel == -1 and groups == 0 and smem >= 2 * rows
