@@ -124,6 +124,9 @@ PlanImpl* plan_steps(const aclfftHandle_t* h, aclfftResult* why)
         adj.kind = Kind::R2C;
         adj.weight = gfft::WEIGHT_STORE_X2;
     }
+    // a tuned choice of no codelets was timed on the primary transform; the
+    // adjoint keeps its codelet, which the weighted entry needs
+    if (pr.kind != Kind::C2C && adj.hints.codelets == 0) adj.hints.codelets = -1;
     bool ok = true;
     for (int v = 0; v < 4 && ok; ++v) {
         int64_t ws = 0, ws2 = 0;

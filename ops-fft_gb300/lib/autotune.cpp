@@ -108,7 +108,7 @@ std::string signature(const StepList& sl)
         switch (s.kind) {
         case Step::ROW:
             os << s.row.codelet << ',' << s.row.ngroups << ',' << s.row.nstage << ',' << s.row.nbuf << ','
-               << s.row.tfpc << ',' << s.has_dev << ',';
+               << s.row.tfpc << ',' << s.row.tile << s.has_dev << ',';
             for (int p = 0; p < s.row.ip.npass; ++p) os << s.row.ip.pass[p].radix << '.';
             break;
         case Step::COL:

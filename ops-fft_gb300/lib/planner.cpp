@@ -414,7 +414,16 @@ bool make_codelet_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, in
             }
         }
     }
-    if (best_ng == 0) return false;
+    if (best_ng == 0) {
+        // a tuned shape that this transform has no room for (it was timed on
+        // another: the adjoint's slots are one bin longer): the score's choice
+        if (!t_hints || (t_hints->codelet_ng <= 0 && t_hints->codelet_nst <= 0 && t_hints->codelet_pp < 0)) return false;
+        PlanHints free = *t_hints;
+        free.codelet_ng = free.codelet_nst = 0;
+        free.codelet_pp = -1;
+        const HintScope scope(&free);
+        return make_codelet_step(L, ntf, in_dist, out_dist, io_mode, nreal, weight, tb, st);
+    }
     tb = trial;
     st.post_off = post_off;
     a.ntf = ntf;

@@ -67,3 +67,47 @@ def test_no_codelets_means_the_generic_row_kernel():
     assert r.returncode == 0, r.stderr[-2000:]
     for check, kernel, groups, smem, rows in json.loads(r.stdout.strip().splitlines()[-1]):
         assert check == "ok" and kernel == -1 and groups == 0 and smem >= 2 * rows
+
+
+_WEIGHTED = r"""
+import sys
+sys.path[:0] = [sys.argv[1] + "/ops-fft_gb300", sys.argv[1] + "/oracle"]
+import numpy as np, torch, aclfft as A, oracle as O
+n, b = 1024, 64
+rng = np.random.default_rng(n)
+X = (rng.standard_normal((b, n // 2 + 1)) + 1j * rng.standard_normal((b, n // 2 + 1))).astype(np.complex64)
+w = rng.random((b, n // 2 + 1), dtype=np.float32)
+with A.Plan.plan1d(n, A.R2C, b) as p:
+    p.set_autotune(True)
+    assert p.info().tuned == 1 and p.check() == "ok"
+    print("candidates", p.info().tune_candidates)
+    Xd, wd, gd = torch.from_numpy(X).cuda(), torch.from_numpy(w).cuda(), torch.empty((b, n), device="cuda")
+    torch.cuda.synchronize()
+    p.exec_r2c_adjoint_weighted(Xd, wd, gd)
+    torch.cuda.synchronize()
+half = np.full(n // 2 + 1, 0.5)
+half[0] = half[-1] = 1.0
+e = O.errors(gd.cpu().numpy(), O.c2r((X * w * half).astype(np.complex128), n))
+assert e["rel_l2"] <= 1e-6, e
+"""
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("choice", ["-1 0 0 0 -1 0 -1", "-1 15 4 -1 -1 0 1"])
+def test_weighted_adjoint_of_a_tuned_plan(choice, tmp_path):
+    """Whatever tuning chose for the R2C itself, its weighted adjoint runs as it
+    did before tuning: after a tuning of its own, and with cached choices of no
+    codelets and of a codelet shape that does not fit shared memory."""
+    pytest.importorskip("torch")
+    path = tmp_path / "plan_tune.txt"
+    env = dict(os.environ, OPS_FFT_PLAN_TUNE_CACHE=str(path))
+
+    def child():
+        r = subprocess.run([sys.executable, "-c", _WEIGHTED, ROOT], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return r.stdout
+
+    child()
+    key = path.read_text().splitlines()[-1].split()[0]
+    path.write_text(f"{key} {choice}\n")
+    assert "candidates 0" in child()
