@@ -11,7 +11,9 @@
 // Choices are cached per (device, kind, length, batch, layout) for the
 // process and, when OPS_FFT_PLAN_TUNE_CACHE names a file, across processes
 // (one line per key; a line that does not parse is ignored, so a damaged
-// file only costs a re-tune).
+// file only costs a re-tune).  A key starts with the version of the kernels
+// that were timed: lines of another version are choices among other launches
+// and are neither used nor kept.
 //
 // The reference has no tuner: its radix choices are fixed tables
 // (src/common/host/fft_exec_helper.h:76-139).
@@ -33,6 +35,9 @@ namespace {
 std::mutex g_mu;
 std::map<std::string, PlanHints> g_cache;
 bool g_file_loaded = false;
+
+// Raised when the candidates or the kernels behind them change.
+constexpr char kCacheVersion[] = "v2:";
 
 const char* cache_path()
 {
@@ -56,6 +61,7 @@ void load_file()
         if (!(is >> key >> h.codelet_variant >> h.codelet_ng >> h.codelet_nst >> h.codelets >> h.cluster >>
               h.cluster_c >> h.codelet_pp))
             continue;
+        if (key.compare(0, sizeof kCacheVersion - 1, kCacheVersion) != 0) continue;
         if (h.codelet_variant < -1 || h.codelet_variant > 64 || h.codelet_ng < 0 || h.codelet_ng > 15 ||
             h.codelet_nst < 0 || h.codelet_nst > 4 || h.codelets < -1 || h.codelets > 1 || h.cluster < -1 ||
             h.cluster > 1 || (h.cluster_c != 0 && h.cluster_c != 2 && h.cluster_c != 4 && h.cluster_c != 8 &&
@@ -92,7 +98,7 @@ std::string cache_key(const aclfftHandle_t* h)
     for (char& c : name)
         if (c == ' ') c = '_';
     std::ostringstream os;
-    os << name << ':' << prop.multiProcessorCount << ':' << (int)h->type << ':' << h->rank << ':' << h->lengths[0]
+    os << kCacheVersion << name << ':' << prop.multiProcessorCount << ':' << (int)h->type << ':' << h->rank << ':' << h->lengths[0]
        << ':' << (h->rank >= 2 ? h->lengths[1] : 1) << ':' << (h->rank == 3 ? h->lengths[2] : 1) << ':' << h->batch
        << ':' << h->stride[0] << ':' << h->precision;
     return os.str();

@@ -111,3 +111,33 @@ def test_weighted_adjoint_of_a_tuned_plan(choice, tmp_path):
     key = path.read_text().splitlines()[-1].split()[0]
     path.write_text(f"{key} {choice}\n")
     assert "candidates 0" in child()
+
+
+_TUNE_PLAN = r"""
+import sys
+sys.path[:0] = [sys.argv[1] + "/ops-fft_gb300"]
+import aclfft as A
+with A.Plan.plan1d(1024, A.R2C, 512) as p:
+    p.set_autotune(True)
+    print("candidates", p.info().tune_candidates)
+"""
+
+def _run_child(code, **env):
+    r = subprocess.run([sys.executable, "-c", code, ROOT], env=dict(os.environ, **env), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return r.stdout
+
+
+@pytest.mark.gpu
+def test_plan_choices_of_other_kernels_are_not_used(tmp_path):
+    """A tune file written before the launches changed has no version: it is
+    tuned again, and the file then holds lines that are used."""
+    pytest.importorskip("torch")
+    path = tmp_path / "plan_tune.txt"
+    env = {"OPS_FFT_PLAN_TUNE_CACHE": str(path)}
+    _run_child(_TUNE_PLAN, **env)
+    line = path.read_text().splitlines()[-1]
+    path.write_text(line.split(":", 1)[1] + "\n" if line.startswith("v") else line + "\n")
+    assert "candidates 0" not in _run_child(_TUNE_PLAN, **env)
+    assert "candidates 0" in _run_child(_TUNE_PLAN, **env)
