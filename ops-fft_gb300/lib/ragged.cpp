@@ -12,7 +12,8 @@
 // Autotuning: per class, candidate radix orders are timed in isolation on
 // scratch buffers and the fastest is kept; choices are
 // cached process-wide (and in a text file when OPS_FFT_TUNE_CACHE names
-// one) keyed by (kind, length).
+// one) keyed by (kind, length), as the radices of the one or two transforms:
+// radices that are no candidate of a length any more are tuned again.
 //
 // Execution: the kernel launch (its last CTA leaves the queue cleared for the
 // next one), captured once per (input, output, direction) into a CUDA graph
@@ -124,9 +125,11 @@ struct Choice {
 };
 
 std::mutex g_tune_mu;
-std::map<Key, Choice> g_tuned;
+std::map<Key, std::string> g_tuned;  // tuned radices, see radices_text
 bool g_tune_file_loaded = false;
 
+// File lines: "r <kind> <length> <radices>", e.g. "r 0 8192 16.8+8.8"; any
+// other line is ignored.
 void load_tune_file()
 {
     if (g_tune_file_loaded) return;
@@ -134,8 +137,13 @@ void load_tune_file()
     const char* path = std::getenv("OPS_FFT_TUNE_CACHE");
     if (!path || !*path) return;
     std::ifstream f(path);
-    int t, n, a, b;
-    while (f >> t >> n >> a >> b) g_tuned[{t, n}] = {a, b};
+    std::string line;
+    while (std::getline(f, line)) {
+        std::istringstream is(line);
+        std::string tag, radices;
+        int t, n;
+        if ((is >> tag >> t >> n >> radices) && tag == "r") g_tuned[{t, n}] = radices;
+    }
 }
 
 void save_tune_file()
@@ -143,7 +151,7 @@ void save_tune_file()
     const char* path = std::getenv("OPS_FFT_TUNE_CACHE");
     if (!path || !*path) return;
     std::ofstream f(path, std::ios::trunc);
-    for (auto& kv : g_tuned) f << kv.first.type << ' ' << kv.first.n << ' ' << kv.second.v1 << ' ' << kv.second.v2 << '\n';
+    for (auto& kv : g_tuned) f << "r " << kv.first.type << ' ' << kv.first.n << ' ' << kv.second << '\n';
 }
 
 struct ClassPlan {
@@ -279,6 +287,31 @@ bool apply_choice(ClassPlan& cp, Choice ch)
     }
     cp.choice = ch;
     return class_smem(c) <= kSmemBudget;
+}
+
+// The radices of a choice: "16.16.16", of a long transform "16.8+8.8".
+std::string radices_text(const ClassPlan& cp, Choice ch)
+{
+    std::ostringstream os;
+    auto put = [&](const TilePlan& t) {
+        for (int q = 0; q < t.np; ++q) os << (q ? "." : "") << t.pass[q].radix;
+    };
+    put(cp.cand1[ch.v1]);
+    if (cp.dev.mode == RAG_MODE_LONG) {
+        os << '+';
+        put(cp.cand2[ch.v2]);
+    }
+    return os.str();
+}
+
+// Applies the choice with these radices; false when there is none any more.
+bool apply_radices(ClassPlan& cp, const std::string& radices)
+{
+    const int n2 = cp.dev.mode == RAG_MODE_LONG ? (int)cp.cand2.size() : 1;
+    for (int a = 0; a < (int)cp.cand1.size(); ++a)
+        for (int b = 0; b < n2; ++b)
+            if (radices_text(cp, {a, b}) == radices) return apply_choice(cp, {a, b});
+    return false;
 }
 
 double class_cost(const RagClass& c) { return (double)c.L * std::log2((double)std::max(c.L, 2)); }
@@ -565,7 +598,7 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
         ClassPlan& cp = p->classes[ci];
         const Key key{cp.dev.type, cp.dev.n};
         auto hit = g_tuned.find(key);
-        if (hit != g_tuned.end() && apply_choice(cp, hit->second)) {
+        if (hit != g_tuned.end() && apply_radices(cp, hit->second)) {
             cp.tuned = true;
             continue;
         }
@@ -649,7 +682,7 @@ aclfftResult autotune(aclfftRaggedPlan_t* p)
         if (!ok) break;
         apply_choice(cp, bestc);
         cp.tuned = true;
-        g_tuned[key] = bestc;
+        g_tuned[key] = radices_text(cp, bestc);
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);

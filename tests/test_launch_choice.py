@@ -122,6 +122,26 @@ with A.Plan.plan1d(1024, A.R2C, 512) as p:
     print("candidates", p.info().tune_candidates)
 """
 
+_TUNE_RAGGED = r"""
+import sys
+sys.path[:0] = [sys.argv[1] + "/ops-fft_gb300", sys.argv[1] + "/oracle"]
+import numpy as np, torch, aclfft as A, oracle as O
+lens = np.array([1500, 1500, 18000], np.int32)
+kinds = np.full(3, A.C2C, np.int32)
+ino, outo, ci, co = A.ragged_layout(lens, kinds)
+x = np.random.default_rng(1).standard_normal(ci // 4).astype(np.float32)
+xd, yd = torch.from_numpy(x).cuda(), torch.zeros(co // 4, device="cuda")
+with A.RaggedPlan(lens, kinds, ino, outo) as p:
+    p.set_stream(torch.cuda.current_stream())
+    p.exec(xd, yd, A.FORWARD)
+    assert p.error_flags() == 0 and p.info().tuned_classes == 2
+y = yd.cpu().numpy()
+for n, i, o in zip(lens.tolist(), (ino // 4).tolist(), (outo // 4).tolist()):
+    e = O.errors(y[o:o + 2 * n].view(np.complex64), O.c2c(x[i:i + 2 * n].view(np.complex64)[None], -1)[0])
+    assert e["rel_l2"] <= 1e-6, (n, e)
+"""
+
+
 def _run_child(code, **env):
     r = subprocess.run([sys.executable, "-c", code, ROOT], env=dict(os.environ, **env), capture_output=True, text=True,
                        timeout=300)
@@ -141,3 +161,22 @@ def test_plan_choices_of_other_kernels_are_not_used(tmp_path):
     path.write_text(line.split(":", 1)[1] + "\n" if line.startswith("v") else line + "\n")
     assert "candidates 0" not in _run_child(_TUNE_PLAN, **env)
     assert "candidates 0" in _run_child(_TUNE_PLAN, **env)
+
+
+@pytest.mark.gpu
+def test_ragged_choices_name_their_radices(tmp_path):
+    """A ragged tune file of candidate indices (as written before), one with
+    radices that the length does not have, and one of this version."""
+    pytest.importorskip("torch")
+    path = tmp_path / "ragged_tune.txt"
+    for old in ("0 1500 1 0\n0 18000 1 1\n", "r 0 1500 15.10.9\nr 0 18000 150.120\n"):
+        path.write_text(old)
+        for _ in range(2):  # tuned again, then read back
+            _run_child(_TUNE_RAGGED, OPS_FFT_TUNE_CACHE=str(path))
+            lines = [line.split() for line in path.read_text().splitlines()]
+            assert [line[:3] for line in lines] == [["r", "0", "1500"], ["r", "0", "18000"]], lines
+            for _, _, n, radices in lines:
+                product = 1
+                for r in radices.replace("+", ".").split("."):
+                    product *= int(r)
+                assert product == int(n) and radices.count("+") == int(int(n) > 4096)
