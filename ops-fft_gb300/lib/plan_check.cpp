@@ -69,12 +69,14 @@ int buffers_used(int npass, int start, bool last_global)
 
 // Tile kernel (csrc/tile_fft.cuh): every shared index of every pass, as the
 // kernel computes it, inside the exchange buffer and injective per pass.
+// first_reads: the first pass reads the buffer too (Hermitian pre-process);
+// last_writes: the last one writes it, padded (even/odd post-process).
 bool check_tile(const InnerPlan& ip, int W, int emul, int cmul, int ps, int64_t bufsz, int nbuf, int64_t smem_bytes,
-                bool first_reads, std::string& why)
+                bool first_reads, bool last_writes, std::string& why)
 {
     if (ip.rmax != 16 || W < 1 || W * ip.nthr > 512) return fail(why, "tile threads");
-    if (nbuf != 1 && nbuf != 2) return fail(why, "tile buffers");
-    if (nbuf * bufsz * 8 > smem_bytes || smem_bytes > kMaxSmemBytes) return fail(why, "tile smem");
+    if (nbuf != 1) return fail(why, "tile buffers");
+    if (bufsz * 8 > smem_bytes || smem_bytes > kMaxSmemBytes) return fail(why, "tile smem");
     auto pad = [&](int i) { return i + (i >> ps); };
     const int L = ip.L;
     if (W > 1 && emul == 1 && cmul < pad(L - 1) + 1) return fail(why, "tile pitch");
@@ -87,7 +89,7 @@ bool check_tile(const InnerPlan& ip, int W, int emul, int cmul, int ps, int64_t 
         for (int j = 0; j < nbf; ++j) {
             for (int r = 0; r < R; ++r) {
                 if ((p > 0 || first_reads) && pad(j) + r * (nbf + (nbf >> ps)) != pad(j + r * nbf)) return fail(why, "tile read stride");
-                if (p + 1 < ip.npass) {
+                if (p + 1 < ip.npass || last_writes) {
                     const int i0 = j / ns * ns * R + j % ns, ws = ns == 1 ? 1 : ns + (ns >> ps);
                     if (pad(i0) + r * ws != pad(i0 + r * ns)) return fail(why, "tile write stride");
                 }
@@ -108,7 +110,7 @@ bool check_row(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
         if (a.codelet >= 0 || a.staged || a.host_in) return fail(why, "tile row mode");
         if (a.ntf >= (int64_t(1) << 31) - 64) return fail(why, "tile rows");
         if (!check_tile(a.ip, a.tfpc, 1, a.lpad, a.pshift, (int64_t)a.tfpc * a.lpad, a.nbuf, a.smem_bytes,
-                        a.io_mode == IO_C2R_EVEN, why)) return false;
+                        a.io_mode == IO_C2R_EVEN, a.io_mode == IO_R2C_EVEN, why)) return false;
     } else {
     if (a.codelet < 0 && (a.ip.nthr * a.tfpc > maxthr || a.tfpc < 1)) return fail(why, "row threads");
     if (a.tfpc < 1) return fail(why, "row tile");
@@ -211,7 +213,7 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
             return fail(why, "paired columns mode");
         if (a.cpi != a.pair_m / 2 + 1 || a.ncols < 1 || a.ncols % a.cpi || a.ncols * 2 >= (int64_t(1) << 31) - 64)
             return fail(why, "paired columns");
-        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, !r2c, why)) return false;
+        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, !r2c, r2c, why)) return false;
         const int64_t items = a.ncols / a.cpi;
         if (a.in_stride != a.pair_m || (r2c && a.out_stride != a.pair_m) || (r2c ? a.ons != a.pair_m : a.ons != 1))
             return fail(why, "paired columns strides");
@@ -234,7 +236,7 @@ bool check_col(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
     if (a.tile) {
         if (a.tfpc & (a.tfpc - 1)) return fail(why, "tile column mode");
         if (a.ncols >= (int64_t(1) << 31) - 64) return fail(why, "tile columns");
-        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, false, why)) return false;
+        if (!check_tile(a.ip, a.tfpc, a.tfpc, 1, a.pshift, a.wsize, a.nbuf, a.smem_bytes, false, false, why)) return false;
         if (a.staged_out && (a.spitch < L || (int64_t)a.tfpc * a.spitch > a.wsize)) return fail(why, "tile staging");
     } else {
         const int maxthr = a.ip.rmax == 16 ? 512 : 256;
