@@ -1138,25 +1138,46 @@ bool make_dtile(int64_t n, int64_t ntf, bool t_fast, bool c2r, DPassArgs& a)
     const int ps = tile_pshift((int)n, rad, c2r);
     const int64_t lp = n + (n >> ps);
     int W = 1, threads = 0;
+    // work of a CTA of w transforms in units of a full warp's, and the threads it needs
+    auto cost = [&](int w, int64_t& need) {
+        int64_t c = 0;
+        need = 32;
+        for (int r : rad) {
+            const int64_t nb = r >= kDTileElems ? 1 : kDTileElems / r, bf = w * (n / r);
+            need = std::max(need, ceil_div(bf, nb));
+            c += ceil_div(bf, 32) * r;
+        }
+        need = ceil_div(need, 32) * 32;
+        return (double)c / w;
+    };
+    int64_t need = 0;
     if (t_fast) {
-        // 8 columns (128-byte segments) where the threads allow it
+        // 8 columns (128-byte segments) where the threads allow it, more while
+        // they fill the lanes of their warps better: short axes have few
+        // butterflies a column (us, one launch a radix / 8 columns / this: 2D
+        // Z2Z 500 x 16 x 64 61 / 93 / 48, 100 x 24 x 100 49 / 42 / 35, Z2D
+        // 1551 x 9 x 64 62 / 86 / 46, 49 x 16 x 1305 173 / 218 / 174; 100 x
+        // 48 x 60 stays at 8: 51 / 35, 16 columns 36)
         W = 8;
         while (W > 1 && W * T > kDTileThreads) W >>= 1;
-        threads = (W * T + 31) / 32 * 32;
+        double best = cost(W, need);
+        threads = (int)need;
+        for (int w = 2 * W; W >= 8 && w <= 32 && ntf / w >= 304 && w * lp * 16 <= 72 * 1024; w *= 2) {
+            const double c = cost(w, need);
+            if (need > kDTileThreads) break;
+            if (c < 0.95 * best) {
+                best = c;
+                W = w;
+                threads = (int)need;
+            }
+        }
     } else {
         // the rows per CTA whose passes fill the lanes of their warps best
         // (a tie goes to fewer; few transforms keep one row a CTA)
         double best = 0;
         for (int w = 1; w * T <= kDTileThreads + 31 && w <= 64 && w * (lp | 1) * 16 <= 72 * 1024; ++w) {
-            int64_t need = 32, cost = 0;
-            for (int r : rad) {
-                const int64_t nb = r >= kDTileElems ? 1 : kDTileElems / r, bf = w * (n / r);
-                need = std::max(need, ceil_div(bf, nb));
-                cost += ceil_div(bf, 32) * r;
-            }
-            need = (need + 31) / 32 * 32;
+            const double c = cost(w, need);
             if (need > kDTileThreads) break;
-            const double c = (double)cost / w;
             if (threads == 0 || c < 0.98 * best) {
                 best = c;
                 W = w;
