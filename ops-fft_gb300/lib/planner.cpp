@@ -1,5 +1,6 @@
 // planner.cpp - see planner.h.
 #include "planner.h"
+#include "tile_list.h"
 
 #include <algorithm>
 #include <cmath>
@@ -300,6 +301,20 @@ int tile_pshift(int L, const std::vector<int>& rad, bool c2r)
 
 namespace {
 
+// Whether a tile is compiled in with its length, threads and radices.
+bool tile_compiled(bool rows, int L, int T, int W, const std::vector<int>& rad)
+{
+#define GFFT_IS_ROW(ID, LL, TT, WW, ...) \
+    if (rows && L == LL && T == TT && W == WW && rad == std::vector<int>{__VA_ARGS__}) return true;
+#define GFFT_IS_COL(ID, LL, TT, WW, ...) \
+    if (!rows && L == LL && T == TT && W == WW && rad == std::vector<int>{__VA_ARGS__}) return true;
+    GFFT_TILE_ROWS(GFFT_IS_ROW)
+    GFFT_TILE_COLS(GFFT_IS_COL)
+#undef GFFT_IS_ROW
+#undef GFFT_IS_COL
+    return false;
+}
+
 // Score bonus of a codelet configuration with a per-group work buffer
 // (ping-pong passes) over the in-place one.
 constexpr double kPingPongScore = 0.0;
@@ -514,8 +529,11 @@ bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, i
     }
     // two warps per CTA, more only for longer rows: small CTAs wait for
     // fewer threads at each barrier (100 x 131072: 36.4 us at 64 threads, 41
-    // at 256; 1024 x 16384: 44.3 against 48.0)
-    const int W = (int)std::max<int64_t>(1, std::min<int64_t>(64 / T, ntf));
+    // at 256; 1024 x 16384: 44.3 against 48.0).  With fewer rows than that a
+    // compiled tile keeps its width and idles (one row, us: R2C 256 3.7 -> 2.1,
+    // codelet 2.9; C2C 128 2.4 -> 1.5)
+    const int full = std::max(1, 64 / T);
+    const int W = tile_compiled(true, L, T, full, rad) ? full : (int)std::min<int64_t>(full, ntf);
     const int64_t one = (int64_t)W * pitch * 8;
     if (one > kMaxSmemBytes) return false;
     tb = trial;

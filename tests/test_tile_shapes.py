@@ -73,3 +73,38 @@ def test_planner_arrives_at_the_shape(ident, rows, L, T, W, rad):
             if i.onchip_length == L:
                 found.append((i.threads_per_transform, i.transforms_per_cta, [i.radix[k] for k in range(i.nradix)]))
     assert (T, W, rad) in found, found
+
+
+@pytest.mark.parametrize("n,typ,rad,T,W", [(256, A.R2C, [16, 8], 16, 4), (128, A.C2C, [16, 8], 16, 4),
+                                           (256, A.C2C, [16, 16], 16, 4), (512, A.C2C, [8, 8, 8], 64, 1)])
+@pytest.mark.parametrize("b", [1, 2, 3, 5])
+def test_few_rows_take_a_compiled_tile(n, typ, rad, T, W, b):
+    with A.Plan.plan1d(n, typ, b) as p:
+        assert p.check() == "ok"
+        i = p.info()
+        assert ([i.radix[k] for k in range(i.nradix)], i.threads_per_transform, i.transforms_per_cta) == (rad, T, W)
+    L = int(np.prod(rad))
+    assert any(s[1] and (s[2], s[3], s[4], s[5]) == (L, T, W, rad) for s in SHAPES)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 15, 64, 128, 256, 300, 512, 1024])
+@pytest.mark.parametrize("b", [1, 3])
+def test_rows_that_leave_most_of_a_tile_idle(n, b):
+    """Tolerance: twice 2^-24 per radix-2 level, one product and one sum each."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((b, n)) + 1j * rng.standard_normal((b, n))).astype(np.complex64)
+    bound = 2.0 * 2.0 ** -24 * max(np.log2(n), 2.0)
+    st = torch.cuda.current_stream()
+    with A.Plan.plan1d(n, A.C2C, b) as p, A.Plan.plan1d(n, A.R2C, b) as q, A.Plan.plan1d(n, A.C2R, b) as c:
+        for plan in (p, q, c):
+            plan.set_stream(st)
+        xd, rd = torch.from_numpy(x).cuda(), torch.from_numpy(x.real.copy()).cuda()
+        hd, bd = torch.empty((b, n // 2 + 1), dtype=torch.complex64, device="cuda"), torch.empty_like(rd)
+        p.exec_c2c(xd, xd, A.FORWARD)  # in place
+        q.exec_r2c(rd, hd)
+        c.exec_c2r(hd, bd)
+    h = np.fft.rfft(x.real.astype(np.float64))
+    for out, exact in ((xd, np.fft.fft(x.astype(np.complex128))), (hd, h), (bd, x.real.astype(np.float64) * n)):
+        assert np.linalg.norm(out.cpu().numpy() - exact) <= 2 * bound * np.linalg.norm(exact)
