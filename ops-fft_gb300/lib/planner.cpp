@@ -503,10 +503,11 @@ bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, i
     if (rad.empty()) return false;
     int T = tile_threads(L, rad);
     if (T > kTileMaxThreads) return false;
-    // one thread per row reads 8 L bytes of its own: beyond 12 complex
-    // values the row kernel's staged copies are faster (16 x 2^20: 100 against
-    // 129 us; 12 x 1.4M: 84 against 81)
-    if (T == 1 && L > 12 && io_mode == IO_C2C) return false;
+    // one thread per row reads 8 L bytes of its own: beyond 12 complex values
+    // and 12 MB the row kernel's staged copies are faster (us, row kernel /
+    // this: 16 x 2^20 100 / 129, x 131072 17.0 / 18.4, x 100000 16.0 / 15.1, x
+    // 1000 4.3 / 2.9; 13 x 100000 11.3 / 9.7; 12 x 1.4M 81 / 84)
+    if (T == 1 && L > 12 && io_mode == IO_C2C && ntf * L > 3 << 19) return false;
     // few rows: one butterfly a thread and pass (half the instructions on a
     // row's critical path when its radices are 8 or less) while that leaves
     // at most 256 threads on an SM

@@ -108,3 +108,32 @@ def test_rows_that_leave_most_of_a_tile_idle(n, b):
     h = np.fft.rfft(x.real.astype(np.float64))
     for out, exact in ((xd, np.fft.fft(x.astype(np.complex128))), (hd, h), (bd, x.real.astype(np.float64) * n)):
         assert np.linalg.norm(out.cpu().numpy() - exact) <= 2 * bound * np.linalg.norm(exact)
+
+
+@pytest.mark.parametrize("n", [13, 14, 15, 16])
+def test_one_thread_rows_up_to_12_mb(n):
+    line = (3 << 19) // n
+    for b, stages in ((1, 1), (line, 1), (line + 1, 2)):  # tiles have one stage, the row kernel prefetches
+        with A.Plan.plan1d(n, A.C2C, b) as p:
+            assert p.check() == "ok"
+            assert min(p.info().stages, 2) == stages
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [13, 14, 15, 16])
+def test_one_thread_rows(n):
+    """One row, a tile that is not full, and both sides of the kernels' line.
+    Tolerance: twice 2^-24 per radix-2 level."""
+    torch = pytest.importorskip("torch")
+    for b in (1, 65, (3 << 19) // n, (3 << 19) // n + 1):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(n + b)
+        x = torch.randn((b, n), dtype=torch.complex64, generator=g, device="cuda")
+        exact = torch.fft.fft(x.to(torch.complex128))
+        y = torch.empty_like(x)
+        with A.Plan.plan1d(n, A.C2C, b) as p:
+            p.set_stream(torch.cuda.current_stream())
+            p.exec_c2c(x, y, A.FORWARD)
+            p.exec_c2c(x, x, A.FORWARD)  # in place
+        assert ((y - exact).norm() / exact.norm()).item() <= 2.0 * 2.0 ** -24 * np.log2(n)
+        assert torch.equal(x, y)
