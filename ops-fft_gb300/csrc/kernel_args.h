@@ -90,7 +90,8 @@ struct RowArgs {
     int32_t host_in;
     // register-to-register rows of any length with radices <= 16
     // (csrc/tile_fft.cuh): tfpc rows per CTA, one exchange buffer of
-    // tfpc * lpad float2 or two (nbuf); twiddles are read from global memory
+    // tfpc * lpad float2 (nbuf 1); twiddles are read from global memory.  2: on
+    // the kernel that the plan's modes share unless the tile is compiled in
     int32_t tile;
 };
 
@@ -126,8 +127,8 @@ struct ColArgs {
     float scale;
     int32_t smem_bytes;
     // register-to-register tiles of any length with radices <= 16
-    // (csrc/tile_fft.cuh): tfpc columns per CTA, exchange buffers (nbuf) of
-    // wsize float2, padded by one element every 2^pshift; with otw2d the
+    // (csrc/tile_fft.cuh; 2 as in RowArgs): tfpc columns per CTA, one exchange
+    // buffer (nbuf 1) of wsize float2, padded by one element every 2^pshift; with otw2d the
     // outer twiddles W^{j*(jb + r*L/R)} are otw_hi[jb*ons + j] * otw_lo[r*ons + j]
     int32_t tile;
     int32_t wsize;

@@ -6,6 +6,7 @@
 #include "tile_list.h"
 
 namespace gfft {
+int launch_tile_any(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
 int launch_tile_io0(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
 int launch_tile_io0w(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
 int launch_tile_io1(const TileArgs& t, int threads, size_t smem, unsigned grid, cudaStream_t st);
@@ -33,7 +34,7 @@ bool shape_is(const TileArgs& t, int L, int T, int W, bool rows, std::initialize
     return t.pshift == (rad.size() > 1 && (1 << k) == *rad.begin() ? k : 30);
 }
 
-int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
+int launch_tile(int io, const TileArgs& t, size_t smem, bool shared, cudaStream_t st)
 {
     int threads = t.W * t.ip.nthr;
     threads = (threads + 31) & ~31;
@@ -55,6 +56,8 @@ int launch_tile(int io, const TileArgs& t, size_t smem, cudaStream_t st)
 #undef GFFT_SHAPE_COL
         if (rc != kNoTileShape) return rc;
     }
+    if (shared && !wide && (io == IO_C2C || io == IO_R2C_EVEN || io == IO_C2R_EVEN))
+        return launch_tile_any(t, threads, smem, grid, st);
     switch (io) {
     case IO_C2C:
         // the span of one transform decides the offset width
@@ -102,7 +105,8 @@ extern "C" int gfft_launch_tile_row(const RowArgs* a, void* stream)
     t.scale = a->scale;
     t.wl = a->wload;
     t.wdist = a->wdist;
-    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
+    t.io = a->io_mode;
+    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, a->tile == 2, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int gfft_launch_tile_col(const ColArgs* a, void* stream)
@@ -157,5 +161,6 @@ extern "C" int gfft_launch_tile_col(const ColArgs* a, void* stream)
         t.weight = a->weight;
         if (t.M < 1 || !t.post) return (int)cudaErrorInvalidValue;
     }
-    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, static_cast<cudaStream_t>(stream));
+    t.io = a->io_mode;
+    return launch_tile(a->io_mode, t, (size_t)a->smem_bytes, a->tile == 2, static_cast<cudaStream_t>(stream));
 }

@@ -47,6 +47,16 @@
 
 namespace gfft {
 
+// Template mode of an argument-driven kernel for C2C and the even real modes in
+// one; TileArgs::io tells which.  Plans whose launches differ in mode (rows and
+// columns, the two passes of a long real transform) take it: a launch then
+// finds the passes that the one before it ran in the instruction caches, where
+// kernels of one mode each are cold every time (us, kernel a mode / this, and
+// before the tiles: 2D R2C 115 x 21 x 120 11.0 / 8.8, 9.8; 1 x 875 x 750 16.5 /
+// 13.0, 14.7; 3D R2C 32 x 30 x 40 13.4 / 10.8, 11.7; R2C 17150 x 4 14.2 / 10.4,
+// 11.3; 100000 x 240 143 / 133, 317).  A lone mode is 2 to 6 % faster on a
+// kernel of its own (C2C 360 x 90000 111 / 115, R2C 2100 x 16384 76 / 80).
+constexpr int IO_TILE = -1;
 constexpr int kTileMaxThreads = 512;  // per CTA; two such CTAs per SM, 64 registers a thread
 
 // n / d for n < 2^31 (host-made, see tile_div)
@@ -88,6 +98,7 @@ struct TileArgs {
     uint32_t M;          // paired columns: columns of an item (see tile_pair)
     int32_t otw_shift;
     int32_t conj_in, conj_out, weight, nreal;
+    int32_t io;  // IO_TILE: the mode
     float scale;
     const float* wl;     // even C2R rows: per-bin input weights (row c at c*wdist), or nullptr
     int64_t wdist;
@@ -399,16 +410,18 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
     const uint32_t c0 = blockIdx.x * (uint32_t)A.W;
     const uint32_t col = c0 + (uint32_t)c.c;
     c.ok = c.c < A.W && c.tid < c.T && col < A.ncols;
-    constexpr bool kEven = IO == IO_R2C_EVEN || IO == IO_C2R_EVEN;
+    constexpr bool kAny = IO == IO_TILE;
+    const int io = kAny ? A.io : IO;
+    const bool paired = !rows && (io == IO_R2C_EVEN || io == IO_C2R_EVEN);
     uint32_t item = 0, pu = 0, pj = 0;
-    if (kEven && !rows) c.ok = tile_pair(A, (uint32_t)c.c, item, pu, pj) && c.tid < c.T;
+    if (paired) c.ok = tile_pair(A, (uint32_t)c.c, item, pu, pj) && c.tid < c.T;
     if (!c.ok) c.c = 0;
     const uint32_t cl = c.ok ? col : 0u;
     c.jm = 0;
     if (rows) {
         c.gi = static_cast<const char*>(A.in) + cl * A.in_dist * (IO == IO_R2C_ODD ? 4 : 8);
         c.go = static_cast<char*>(A.out) + cl * A.out_dist * (IO == IO_C2R_ODD ? 4 : 8);
-    } else if constexpr (kEven) {
+    } else if (paired) {
         if (!c.ok) item = pj = 0;
         c.gi = static_cast<const char*>(A.in) + 8 * (item * A.in_dist + pj);
         c.go = static_cast<char*>(A.out) + 8 * (item * A.out_dist + pj);
@@ -427,11 +440,12 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
     pdl_wait();  // every access below may touch the caller's buffers
     c.off = c.c * A.cmul;
     const int np = ST ? S::NP : A.ip.npass;
-    const bool direct = IO != IO_R2C_EVEN && ((ST && S::ROWS) || !A.staged_out);  // the last pass stores to HBM
-    if constexpr (IO == IO_C2R_EVEN) {
+    const bool direct = io != IO_R2C_EVEN && ((ST && S::ROWS) || !A.staged_out);  // the last pass stores to HBM
+    if constexpr (IO == IO_C2R_EVEN || kAny) {
         // Hermitian pre-process into the exchange buffer, every bin loaded
         // once (see codelet_kernel); the passes then all run from it
-        if (!rows) {
+        if (io != IO_C2R_EVEN) {
+        } else if (!rows) {
             // column u's samples X[u + r*M] and their mirrors X[L - u - r*M]:
             // column M - u, sample Lq-1-r (column 0: its own sample Lq-r;
             // r = 0 pairs DC with Nyquist)
@@ -534,7 +548,7 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
                 });
             }
         }
-        __syncthreads();
+        if (io == IO_C2R_EVEN) __syncthreads();
     }
     if constexpr (ST) {
         sfor<S::NP>([&](auto pp) {
@@ -543,33 +557,34 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             if (P + 1 < S::NP) __syncthreads();
         });
     } else {
-    if (IO == IO_C2R_EVEN) {
-        if (np == 1) {
-            GFFT_TILE_SWITCH(0, false, true)
-        } else {
-            GFFT_TILE_SWITCH(0, false, false)
+        // one copy of the inner passes, of which the first one of a C2R is one
+        int p = 1;
+        if constexpr (IO == IO_C2R_EVEN || kAny) {
+            if (io == IO_C2R_EVEN) p = 0;
         }
-    } else if (np == 1) {
-        GFFT_TILE_SWITCH(0, true, true)
-    } else {
-        GFFT_TILE_SWITCH(0, true, false)
-    }
-    if (np > 1) {
-        __syncthreads();
-        for (int p = 1; p + 1 < np; ++p) {
-            // opaque per pass: otherwise every radix' loop-invariant address
-            // arithmetic is computed ahead of the loop (40 instructions an
-            // element)
-            asm volatile("" : "+r"(c.L), "+r"(c.T), "+r"(c.tid), "+r"(c.em), "+r"(c.ps));
-            GFFT_TILE_SWITCH(p, false, false)
-            __syncthreads();
+        if (p == 1) {
+            if (np == 1) {
+                GFFT_TILE_SWITCH(0, true, true)
+            } else {
+                GFFT_TILE_SWITCH(0, true, false)
+            }
         }
-        GFFT_TILE_SWITCH(np - 1, false, true)
-    }
+        if (np > p) {
+            if (p == 1) __syncthreads();
+            for (; p + 1 < np; ++p) {
+                // opaque per pass: otherwise every radix' loop-invariant
+                // address arithmetic is computed ahead of the loop (40
+                // instructions an element)
+                asm volatile("" : "+r"(c.L), "+r"(c.T), "+r"(c.tid), "+r"(c.em), "+r"(c.ps));
+                GFFT_TILE_SWITCH(p, false, false)
+                __syncthreads();
+            }
+            GFFT_TILE_SWITCH(np - 1, false, true)
+        }
     }
     if (direct) return;
     __syncthreads();
-    if constexpr (IO == IO_C2C || IO == IO_C2R_EVEN) {
+    if constexpr (IO == IO_C2C || IO == IO_C2R_EVEN || kAny) {
         if (A.staged_out) {
             // a column's outputs are contiguous: consecutive threads write
             // consecutive bins, two at a time where aligned
@@ -577,12 +592,12 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             const int lane = threadIdx.x & 31;
             for (int q = threadIdx.x >> 5; q < A.W; q += blockDim.x >> 5) {
                 uint32_t it2 = 0, u = 0, j = 0;
-                if constexpr (IO == IO_C2C) {
+                if (!paired) {
                     if (c0 + q >= A.ncols) break;
                     it2 = tdiv(c0 + q, A.cpi);
                     j = c0 + q - it2 * A.cpi.d;
-                } else {
-                    if (!tile_pair(A, (uint32_t)q, it2, u, j)) continue;
+                } else if (!tile_pair(A, (uint32_t)q, it2, u, j)) {
+                    continue;
                 }
                 float2* g = static_cast<float2*>(A.out) + it2 * A.out_dist + (int64_t)j * c.L;
                 const float2* sq = tsm + q * A.spitch;
@@ -599,9 +614,10 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             }
         }
     }
-    if constexpr (IO == IO_R2C_EVEN) {
+    if constexpr (IO == IO_R2C_EVEN || kAny) {
         // even/odd post-process (see codelet_kernel)
-        if (!rows) {
+        if (io != IO_R2C_EVEN) {
+        } else if (!rows) {
             // bins u + M*kk of column u and their mirrors: column M - u, bin
             // Lq-1-kk (column 0: its own bin Lq-kk; kk = 0 is DC and Nyquist)
             const uint32_t W2 = (uint32_t)A.W >> 1;

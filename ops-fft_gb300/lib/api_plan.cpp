@@ -131,6 +131,7 @@ PlanImpl* plan_steps(const aclfftHandle_t* h, aclfftResult* why)
     for (int v = 0; v < 4 && ok; ++v) {
         int64_t ws = 0, ws2 = 0;
         ok = gfft::build_steps(v < 2 ? pr : adj, (v & 1) != 0, impl->tb, impl->lists[v], ws, ws2);
+        if (ok) gfft::share_tiles(impl->lists[v].steps);
         impl->ws_bytes = std::max<int64_t>(impl->ws_bytes, ws);
         impl->ws2_bytes = std::max<int64_t>(impl->ws2_bytes, ws2);
     }

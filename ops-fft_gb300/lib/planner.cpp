@@ -682,6 +682,12 @@ bool make_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, int io
     return a.smem_bytes <= kMaxSmemBytes;
 }
 
+// Whether the launcher has a compiled instance of an even real column tile.
+bool pair_compiled(bool r2c, int L, int T, int W, const std::vector<int>& rad)
+{
+    return tile_compiled(false, L, T, W, rad) && (r2c ? W == 16 || L == 1024 : W == 8);
+}
+
 // Turns the column pass described by st.col (addresses filled in) into tiles
 // of the tile kernel; false when it does not apply.
 bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilder& tb, Step& st)
@@ -1833,6 +1839,36 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         return true;
     }
     return unsupported("odd real-data length beyond one CTA");
+}
+
+// Argument-driven tiles of different modes in one list share a kernel (IO_TILE
+// in csrc/tile_fft.cuh).
+void share_tiles(std::vector<Step>& steps)
+{
+    auto rad = [](const InnerPlan& ip) {
+        std::vector<int> r;
+        for (int p = 0; p < ip.npass; ++p) r.push_back(ip.pass[p].radix);
+        return r;
+    };
+    auto driven = [&](Step& s, int& io) -> int32_t* {
+        if (s.kind == Step::ROW) {
+            RowArgs& a = s.has_dev ? s.dev : s.row;
+            io = a.io_mode;
+            return a.tile && io <= IO_C2R_EVEN && !tile_compiled(true, a.ip.L, a.ip.nthr, a.tfpc, rad(a.ip)) ? &a.tile : nullptr;
+        }
+        if (s.kind != Step::COL || !s.col.tile) return nullptr;
+        ColArgs& a = s.col;
+        io = a.io_mode;
+        const bool compiled = io == IO_C2C ? tile_compiled(false, a.ip.L, a.ip.nthr, a.tfpc, rad(a.ip))
+                                           : pair_compiled(io == IO_R2C_EVEN, a.ip.L, a.ip.nthr, a.tfpc, rad(a.ip));
+        return compiled ? nullptr : &a.tile;
+    };
+    int modes = 0, io = 0;
+    for (Step& s : steps)
+        if (driven(s, io)) modes |= 1 << io;
+    if ((modes & (modes - 1)) == 0) return;
+    for (Step& s : steps)
+        if (int32_t* tile = driven(s, io)) *tile = 2;
 }
 
 }  // namespace gfft

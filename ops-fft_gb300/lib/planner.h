@@ -136,6 +136,10 @@ struct Problem {
 bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& out, int64_t& ws_bytes,
                  int64_t& ws2_bytes);
 
+// Last step of planning a list: which of its launches share a kernel.
+void share_tiles(std::vector<Step>& steps);
+
+
 // Two column passes of a long batched C2C (length n = L1 * L2): the first
 // writes its whole output to BUF_WS, the second reads BUF_WS and writes
 // BUF_OUT.  False when n does not split into exactly two on-chip factors.
