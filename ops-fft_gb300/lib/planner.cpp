@@ -705,14 +705,18 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     int W = S > 1 ? 16 : 8;
     while (W > 4 && W * T > kTileMaxThreads) W >>= 1;
     if (T * W > kTileMaxThreads) return false;
-    // few columns: narrower tiles until two CTAs per SM are there
-    while (W > 4 && a.ncols / W < 304) W >>= 1;
+    // few columns: narrower tiles until two CTAs per SM are there, but not
+    // below the narrowest compiled one (us, 4 columns argument-driven / compiled:
+    // 2D R2C 25 x 128 x 30 8.0 / 5.4, C2R 10 x 256 x 256 12.2 / 8.2, 1 x 512 x 256
+    // 11.3 / 7.6, C2C 22 x 512 x 100 13.8 / 11.4)
+    auto compiled = [&](int w) { return tile_compiled(false, Lq, T, w, rad); };
+    while (W > 4 && a.ncols / W < 304 && (!compiled(W) || compiled(W / 2))) W >>= 1;
     // and, as for rows, a thread for every butterfly while that leaves at most
     // 256 threads on an SM (us, without / with: 32 x 30 2D 7.1 / 5.3, 32 x 30 x
-    // 40 12.3 / 9.9, one row of 262144 9.9 / 8.6)
+    // 40 12.3 / 9.9)
     int T1 = 1;
     for (int r : rad) T1 = std::max(T1, Lq / r);
-    if (T1 * W <= kTileMaxThreads && a.ncols * T1 <= 152 * 256) T = T1;
+    if (!compiled(W) && T1 * W <= kTileMaxThreads && a.ncols * T1 <= 152 * 256) T = T1;
     TwiddleBuilder trial = tb;
     InnerPlan ip;
     if (!build_inner(Lq, rad, T, trial, ip)) return false;

@@ -137,3 +137,31 @@ def test_one_thread_rows(n):
             p.exec_c2c(x, x, A.FORWARD)  # in place
         assert ((y - exact).norm() / exact.norm()).item() <= 2.0 * 2.0 ** -24 * np.log2(n)
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n,width", [(256, 8), (512, 8), (1024, 8), (2048, 4)])
+def test_few_columns_keep_a_compiled_tile(n, width):
+    for b in (2, 3, 17, 257):  # (one column is one row)
+        with A.Plan.plan1d(n, A.C2C, b, A.VERTICAL) as p:
+            assert p.check() == "ok"
+            i = p.info()
+            key = (n, i.threads_per_transform, i.transforms_per_cta, [i.radix[k] for k in range(i.nradix)])
+            assert i.transforms_per_cta == width and key in [s[2:] for s in SHAPES if not s[1]]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,b", [(256, 1), (256, 17), (512, 3), (512, 129), (1024, 1), (1024, 51), (2048, 2), (2048, 65)])
+def test_few_columns(n, b):
+    """Tolerance: twice 2^-24 per radix-2 level."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + b)
+    x = torch.randn((n, b), dtype=torch.complex64, generator=g, device="cuda")
+    exact = torch.fft.fft(x.to(torch.complex128), dim=0)
+    y = torch.empty_like(x)
+    with A.Plan.plan1d(n, A.C2C, b, A.VERTICAL) as p:
+        p.set_stream(torch.cuda.current_stream())
+        p.exec_c2c(x, y, A.FORWARD)
+        p.exec_c2c(x, x, A.FORWARD)  # in place
+    assert ((y - exact).norm() / exact.norm()).item() <= 2.0 * 2.0 ** -24 * np.log2(n)
+    assert torch.equal(x, y)
