@@ -790,10 +790,19 @@ bool make_pair_steps(int64_t L, int64_t batch, bool r2c, int weight, int src, in
     ColArgs& c = ps.col;
     const int Lq = c.ip.L;
     const std::vector<int> rad = choose_tile_radices(Lq, !r2c);
-    const int T = tile_threads(Lq, rad);
+    int T = tile_threads(Lq, rad);
     int W = r2c ? 16 : 8;
     while (W > 8 && W * T > kTileMaxThreads) W >>= 1;
     if (W * T > kTileMaxThreads) return false;
+    // few pairs, as for few columns in make_tile_col: half the width, a thread
+    // for every butterfly (R2C, us: 30000 x 4 11.7 -> 10.4, 36000 x 1 11.9 -> 10.2)
+    const int64_t pairs = batch * (L / Lq / 2 + 1);
+    if (!pair_compiled(r2c, Lq, T, W, rad)) {
+        while (W > 8 && pairs / (W / 2) < 304) W >>= 1;
+        int T1 = 1;
+        for (int r : rad) T1 = std::max(T1, Lq / r);
+        if (T1 * W <= kTileMaxThreads && 2 * pairs * T1 <= 152 * 256) T = T1;
+    }
     if (!build_inner(Lq, rad, T, trial, c.ip)) return false;
     c.pshift = tile_pshift(Lq, rad, !r2c);
     c.pair_m = (int32_t)(L / Lq);
