@@ -315,6 +315,16 @@ bool tile_compiled(bool rows, int L, int T, int W, const std::vector<int>& rad)
     return false;
 }
 
+// Whether any column tile of this length is compiled in.
+bool column_tile_compiled(int L)
+{
+#define GFFT_IS_LEN(ID, LL, TT, WW, ...) \
+    if (L == LL) return true;
+    GFFT_TILE_COLS(GFFT_IS_LEN)
+#undef GFFT_IS_LEN
+    return false;
+}
+
 // Score bonus of a codelet configuration with a per-group work buffer
 // (ping-pong passes) over the in-place one.
 constexpr double kPingPongScore = 0.0;
@@ -767,7 +777,8 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     return true;
 }
 
-bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st);
+bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st,
+                   bool column_kernel = false);
 
 // The two column passes of a long even real transform (complex length L = Lq
 // * Ns) with the even/odd packing on chip: the last pass of an R2C and the
@@ -842,8 +853,9 @@ bool make_pair_steps(int64_t L, int64_t batch, bool r2c, int weight, int src, in
 // independent columns per item, `items` items `D` apart).  The pass runs the
 // q-th factor Lq of the axis decomposition after a product Ns of earlier
 // factors (outer Stockham pass); Ns == 1 and Lq == n is a plain strided
-// transform.
-bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st)
+// transform.  column_kernel: not on tiles (see build_steps).
+bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st,
+                   bool column_kernel)
 {
     std::vector<int> rad = choose_radices(Lq);
     if (rad.empty()) return false;
@@ -888,7 +900,7 @@ bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64
     a.staged_out = staged_out ? 1 : 0;
     a.scale = 1.f;
     st.tw_off = 0;
-    if (make_tile_col(S, Lq, Ns, staged_out, tb, st)) return true;
+    if (!column_kernel && make_tile_col(S, Lq, Ns, staged_out, tb, st)) return true;
     if (!build_inner(Lq, rad, nthr, tb, a.ip)) return false;
     if (Ns > 1) {
         const int64_t M = Ns * Lq;
@@ -960,7 +972,7 @@ bool row_tile_beats_cluster(int io_mode)
 
 // Strided-axis transform as a list of column passes with buffer routing.
 bool make_axis_steps(int64_t n, int64_t S, int64_t items, int64_t D, int src, int dst, int spare, int cap,
-                     TwiddleBuilder& tb, std::vector<Step>& out, bool& needs_spare)
+                     TwiddleBuilder& tb, std::vector<Step>& out, bool& needs_spare, bool column_kernel = false)
 {
     std::vector<int> fac = split_axis(n, cap);
     if (fac.empty()) return false;
@@ -984,7 +996,7 @@ bool make_axis_steps(int64_t n, int64_t S, int64_t items, int64_t D, int src, in
     int64_t Ns = 1;
     for (int q = 0; q < Q; ++q) {
         Step st;
-        if (!make_col_step(n, S, items, D, fac[q], Ns, tb, st)) return false;
+        if (!make_col_step(n, S, items, D, fac[q], Ns, tb, st, column_kernel)) return false;
         st.src = b[q];
         st.dst = b[q + 1];
         if (st.src == spare || st.dst == spare) needs_spare = true;
@@ -1545,6 +1557,27 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         const int64_t last = dims[nd - 1];
         int64_t outer = p.batch;  // rows along the fastest axis
         for (int a = 0; a + 1 < nd; ++a) outer *= dims[a];
+        // beside rows with a prime above 16, on the generic row kernel, the
+        // strided axes of few points stay on the column kernel: a tile's code is
+        // cold after that kernel's, and the passes are too short to make up for
+        // it.  All axes or none (kernels of three kinds are colder still), none
+        // where a compiled tile waits, and of 2D transforms those of 17 to 90
+        // points (us, tiles / column kernel: 3D 60 x 21 x 19 19.0 / 16.1, 32 x 30 x
+        // 41 24.9 / 22.2, 21 x 125 x 41 27.7 / 25.6, 200 x 60 x 41 30.5 / 28.2, but
+        // 16 x 96 x 38 21.0 / 22.8; 2D 470 x 20 x 41 23.3 / 21.7, 2 x 80 x 86 20.3 /
+        // 18.9, but 1 x 75 x 34 15.4 / 16.1, 1 x 16 x 205 20.1 / 21.3, 1 x 300 x 86
+        // 25.5 / 26.3)
+        const int64_t row_len = p.kind == Kind::C2C || last % 2 ? last : last / 2;
+        const std::vector<int> row_rad = row_len <= row_max_length() ? choose_radices((int)row_len) : std::vector<int>{};
+        bool column_kernel = !row_rad.empty() && *std::max_element(row_rad.begin(), row_rad.end()) > 16 &&
+                             outer * (p.kind == Kind::C2C ? last : last / 2 + 1) <= (int64_t)1 << 18;
+        int strided = 0;
+        for (int a = 0; a + 1 < nd; ++a) strided += dims[a] > 1;
+        for (int a = 0; a + 1 < nd && column_kernel; ++a) {
+            const int64_t n = dims[a];
+            if (n > 1 && (n > cap || column_tile_compiled((int)n) || (strided == 1 && (n <= 16 || n > 90))))
+                column_kernel = false;
+        }
 
         if (p.kind == Kind::C2C) {
             // one transform per axis, fastest first: the first pass reads the
@@ -1563,7 +1596,8 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
                         st.src = cur;
                         st.dst = BUF_OUT;
                         out.steps.push_back(st);
-                    } else if (!make_axis_steps(n, S, items, n * S, cur, BUF_OUT, BUF_WS, cap, tb, out.steps, spare)) {
+                    } else if (!make_axis_steps(n, S, items, n * S, cur, BUF_OUT, BUF_WS, cap, tb, out.steps, spare,
+                                                S > 1 && column_kernel)) {
                         return unsupported("multi-dimensional axis length not decomposable");
                     }
                     cur = BUF_OUT;
@@ -1616,7 +1650,8 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
             for (int a = nd - 2; a >= 0; --a) {
                 const int64_t n = dims[a], S = col_stride(a);
                 if (n == 1) continue;
-                if (!make_axis_steps(n, S, col_items(a), n * S, BUF_OUT, BUF_OUT, BUF_WS, cap, tb, out.steps, spare))
+                if (!make_axis_steps(n, S, col_items(a), n * S, BUF_OUT, BUF_OUT, BUF_WS, cap, tb, out.steps, spare,
+                                     column_kernel))
                     return unsupported("column length not decomposable");
                 if (spare) need_ws(half_bytes);
             }
@@ -1633,7 +1668,8 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
             for (int a = nd - 2; a >= 0; --a) {
                 const int64_t n = dims[a], S = col_stride(a);
                 if (n == 1) continue;
-                if (!make_axis_steps(n, S, col_items(a), n * S, from, BUF_WS2, BUF_WS, cap, tb, out.steps, spare))
+                if (!make_axis_steps(n, S, col_items(a), n * S, from, BUF_WS2, BUF_WS, cap, tb, out.steps, spare,
+                                     column_kernel))
                     return unsupported("column length not decomposable");
                 if (spare) need_ws(half_bytes);
                 from = BUF_WS2;
