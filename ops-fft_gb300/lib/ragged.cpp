@@ -47,6 +47,7 @@ constexpr int kMaxSingle = 4096;         // longest on-chip complex length
 constexpr int64_t kMaxLength = 1 << 24;
 constexpr int kOuterTable = 1 << 16;     // longest length with a whole outer-twiddle table (512 KB)
 constexpr int kPostPairs = 4096;         // bin pairs of one post-process item
+constexpr int kResident = 304;           // CTAs at once: two on each of 152 SMs
 // workspace of one group of long transforms: the next group's first steps
 // are queued between a group's first and second steps, so the workspace in
 // flight is two groups and stays in the L2
@@ -159,6 +160,7 @@ struct ClassPlan {
     std::vector<TilePlan> cand1, cand2;
     Choice choice;
     bool tuned = false;
+    int split = 1;             // long: least items a step is cut into, see split_steps
     std::vector<int> members;  // transform indices
 };
 
@@ -282,8 +284,9 @@ bool apply_choice(ClassPlan& cp, Choice ch)
         if (ch.v2 < 0 || ch.v2 >= (int)cp.cand2.size()) return false;
         c.p2 = cp.cand2[ch.v2];
         c.pitch = c.La | 1;  // consecutive columns in different banks
-        c.group = spread_tile(c.p1, std::min(kThreads / c.p1.T, c.Lb), c.Lb);
-        c.group2 = spread_tile(c.p2, std::min(kThreads / c.p2.T, c.La), c.La);
+        auto cut = [&](int cols) { return (cols + cp.split - 1) / cp.split; };
+        c.group = spread_tile(c.p1, std::min(kThreads / c.p1.T, cut(c.Lb)), c.Lb);
+        c.group2 = spread_tile(c.p2, std::min(kThreads / c.p2.T, cut(c.La)), c.La);
     }
     cp.choice = ch;
     return class_smem(c) <= kSmemBudget;
@@ -435,6 +438,33 @@ void build_items(aclfftRaggedPlan_t* p)
     for (auto& s : singles) p->items.push_back(s.second);
     p->smem = 16;
     for (auto& cp : p->classes) p->smem = std::max(p->smem, class_smem(cp.dev));
+}
+
+// Items of a plan that leaves CTAs idle: each step of its long transforms is cut
+// into at least four (else two) items while all still have a CTA of their own.
+// One 512-thread tile holds a whole step of 8192 points, and the two steps wait
+// for each other (us, uncut / cut, and before the tiles: 163 transforms of up to
+// 8192 points 20.7 / 18.8, 17.1; 10 of them 15.9 / 14.8, 14.8; 20 of 8192 19.6 /
+// 16.5, 16.7; 250 22.6 / 18.8, 18.5; into eight: 20 of 8192 19.3, 60 of up to
+// 32768 23.2 against 21.2 uncut).
+void split_steps(aclfftRaggedPlan_t* p)
+{
+    auto build = [&](int split) {
+        for (auto& cp : p->classes) {
+            if (cp.dev.mode != RAG_MODE_LONG) continue;
+            cp.split = split;
+            apply_choice(cp, cp.choice);
+        }
+        build_items(p);
+    };
+    build_items(p);
+    const bool any = std::any_of(p->classes.begin(), p->classes.end(),
+                                 [](const ClassPlan& cp) { return cp.dev.mode == RAG_MODE_LONG; });
+    if (!any || (int)p->items.size() >= kResident) return;
+    for (int split : {4, 2, 1}) {
+        build(split);
+        if ((int)p->items.size() <= kResident) return;
+    }
 }
 
 template <class T>
@@ -877,7 +907,7 @@ ACLFFT_API aclfftResult aclfftRaggedPlanCreate(aclfftRaggedPlan* plan, int count
         gfft::set_last_error("ragged batches: twiddle tables too large");
         return ACLFFT_NOT_SUPPORTED;
     }
-    build_items(p);
+    split_steps(p);
     *plan = p;
     return ACLFFT_SUCCESS;
 }
