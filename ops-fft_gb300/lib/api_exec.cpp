@@ -349,6 +349,20 @@ bool host_direct(const StepList& sl, const void* in, const void* out, size_t in_
            reinterpret_cast<uintptr_t>(*dout) % out_align == 0;
 }
 
+// Whether chunks pay (exec_host_pipelined).  A copy from pageable memory holds
+// the host until it is staged, and one to it until it is done, so chunks then
+// overlap nothing, or with a pinned input only the kernels, which pays on large
+// calls (us, chunks / one copy each way: both pageable C2C 8192 x 64 204 / 98,
+// 4096 x 2048 888 / 786; pageable input 4096 x 256 166 / 132; pageable output
+// 4096 x 256 172 / 121, 2310 x 2000, 70 MB, 423 / 424, 4096 x 2048, 128 MB, 616 /
+// 727; both pinned 4096 x 2048 535 / 725).
+constexpr size_t kPageableOutBytes = 64u << 20;
+
+bool chunks_pay(const void* in, const void* out, size_t in_bytes, size_t out_bytes)
+{
+    return mapped_host(in) && (mapped_host(out) || in_bytes + out_bytes >= kPageableOutBytes);
+}
+
 struct CallShape {
     size_t in_bytes;
     size_t out_bytes;
@@ -437,7 +451,8 @@ aclfftResult exec_common(aclfftHandle_t* h, int variant, void* in, void* out, Ca
     }
     void* dev_in = din ? in : impl->stage_a;
     void* dev_out = dout ? out : impl->stage_b;
-    if (!din && !dout && primary.steps.size() == 1 && primary.steps[0].kind == Step::ROW) {
+    if (!din && !dout && primary.steps.size() == 1 && primary.steps[0].kind == Step::ROW &&
+        chunks_pay(in, out, shape.in_bytes, shape.out_bytes)) {
         const int rc = exec_host_pipelined(impl, primary.steps[0], in, out, shape.in_bytes, shape.out_bytes, st, c2c,
                                            inverse, (float)scale);
         if (rc > 0) return ACLFFT_EXEC_FAILED;
