@@ -192,10 +192,6 @@ int row_nbuf(int npass, int start, bool last_global)
 // Hints of the problem being planned (set by build_steps for its duration).
 thread_local const PlanHints* t_hints = nullptr;
 
-// Plans without tiles (set for its duration): the allocation-free path, whose
-// twiddles live in a fixed array.
-thread_local bool t_no_tiles = false;
-
 struct HintScope {
     explicit HintScope(const PlanHints* h) : prev(t_hints) { t_hints = h; }
     ~HintScope() { t_hints = prev; }
@@ -703,7 +699,7 @@ bool pair_compiled(bool r2c, int L, int T, int W, const std::vector<int>& rad)
 bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilder& tb, Step& st)
 {
     ColArgs& a = st.col;
-    if (a.ncols >= kTileMaxCols || t_no_tiles) return false;
+    if (a.ncols >= kTileMaxCols) return false;
     const std::vector<int> rad = choose_tile_radices(Lq);
     if (rad.empty()) return false;
     int T = tile_threads(Lq, rad);
@@ -853,7 +849,8 @@ bool make_pair_steps(int64_t L, int64_t batch, bool r2c, int weight, int src, in
 // independent columns per item, `items` items `D` apart).  The pass runs the
 // q-th factor Lq of the axis decomposition after a product Ns of earlier
 // factors (outer Stockham pass); Ns == 1 and Lq == n is a plain strided
-// transform.  column_kernel: not on tiles (see build_steps).
+// transform.  column_kernel: not on tiles (see build_steps; and the allocation-
+// free path, whose twiddles live in a fixed array).
 bool make_col_step(int64_t n, int64_t S, int64_t items, int64_t D, int Lq, int64_t Ns, TwiddleBuilder& tb, Step& st,
                    bool column_kernel)
 {
@@ -1068,11 +1065,9 @@ bool build_scratch_c2c_steps(int64_t n, int64_t batch, TwiddleBuilder& tb, std::
     const std::vector<int> fac = split_axis(n, col_max_length());
     if (fac.size() != 2) return false;
     Step first, second;
-    t_no_tiles = true;
-    const bool ok = make_col_step(n, 1, batch, n, fac[0], 1, tb, first) &&
-                    make_col_step(n, 1, batch, n, fac[1], fac[0], tb, second);
-    t_no_tiles = false;
-    if (!ok) return false;
+    if (!make_col_step(n, 1, batch, n, fac[0], 1, tb, first, true) ||
+        !make_col_step(n, 1, batch, n, fac[1], fac[0], tb, second, true))
+        return false;
     first.src = BUF_IN;
     first.dst = BUF_WS;
     second.src = BUF_WS;
