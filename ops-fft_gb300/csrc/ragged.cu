@@ -62,8 +62,7 @@ struct RagCtx {
 
 // One pass (see tile_pass): up to 16 / R butterflies a thread.
 template <int R, bool FIRST, bool LAST>
-__device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int p, const float2* src, float2* dst,
-                                         bool to_global)
+__device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int p, float2* buf, bool to_global)
 {
     constexpr int NB = R >= 16 ? 1 : 16 / R;
     const int nbf = c.L / R;
@@ -135,7 +134,7 @@ __device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int 
         sfor<NB>([&](auto bb) {
             constexpr int b = decltype(bb)::value;
             const int j = min(c.tid + b * c.T, nbf - 1);  // clamped, not guarded: see tile_pass
-            const float2* s = src + (j + (j >> c.ps)) * c.em;
+            const float2* s = buf + (j + (j >> c.ps)) * c.em;
             sfor<R>([&](auto rr) {
                 constexpr int r = decltype(rr)::value;
                 v[b * R + r] = s[r * rs];
@@ -161,7 +160,7 @@ __device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int 
             if (!LAST || !to_global) {
                 int base, ws;
                 if (LAST && q.kind == RAG_P1) {
-                    base = c.c * q.pitch + j - c.c;  // dst already points at column c
+                    base = c.c * q.pitch + j - c.c;  // buf already points at column c
                     ws = ns;
                 } else {
                     const int i0 = qq * ns * R + k;
@@ -170,7 +169,7 @@ __device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int 
                 }
                 sfor<R>([&](auto rr) {
                     constexpr int r = decltype(rr)::value;
-                    dst[base + r * ws] = v[b * R + r];
+                    buf[base + r * ws] = v[b * R + r];
                 });
             } else {
                 char* g = c.go + (uint32_t)j * c.out_st;
@@ -196,7 +195,7 @@ __device__ __forceinline__ void rag_pass(const RagItem& q, const RagCtx& c, int 
 }
 
 #define GFFT_RAG_CASE(RV, P, FIRST, LAST) \
-    case RV: rag_pass<RV, FIRST, LAST>(q, c, P, buf, buf, direct); break;
+    case RV: rag_pass<RV, FIRST, LAST>(q, c, P, buf, direct); break;
 #define GFFT_RAG_SWITCH(P, FIRST, LAST)   \
     switch (q.pass[P].radix) {            \
         GFFT_RAG_CASE(1, P, FIRST, LAST)  \

@@ -101,7 +101,6 @@ extern "C" int gfft_launch_tile_row(const RowArgs* a, void* stream)
     t.conj_in = a->conj_in;
     t.conj_out = a->conj_out;
     t.weight = a->weight;
-    t.nreal = a->nreal;
     t.scale = a->scale;
     t.wl = a->wload;
     t.wdist = a->wdist;

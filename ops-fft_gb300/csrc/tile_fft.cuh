@@ -97,7 +97,7 @@ struct TileArgs {
     int32_t spitch;      // staged_out: shared pitch of one column
     uint32_t M;          // paired columns: columns of an item (see tile_pair)
     int32_t otw_shift;
-    int32_t conj_in, conj_out, weight, nreal;
+    int32_t conj_in, conj_out, weight;
     int32_t io;  // IO_TILE: the mode
     float scale;
     const float* wl;     // even C2R rows: per-bin input weights (row c at c*wdist), or nullptr
@@ -557,21 +557,20 @@ __global__ void __launch_bounds__(MAXT, MINB) tile_kernel(const __grid_constant_
             if (P + 1 < S::NP) __syncthreads();
         });
     } else {
-        // one copy of the inner passes, of which the first one of a C2R is one
-        int p = 1;
+        // the first pass of a C2R reads the exchange buffer, as the inner ones do
+        int first = 1;
         if constexpr (IO == IO_C2R_EVEN || kAny) {
-            if (io == IO_C2R_EVEN) p = 0;
+            if (io == IO_C2R_EVEN) first = 0;
         }
-        if (p == 1) {
-            if (np == 1) {
-                GFFT_TILE_SWITCH(0, true, true)
-            } else {
-                GFFT_TILE_SWITCH(0, true, false)
-            }
+        if (first == 0) {
+        } else if (np == 1) {
+            GFFT_TILE_SWITCH(0, true, true)
+        } else {
+            GFFT_TILE_SWITCH(0, true, false)
         }
-        if (np > p) {
-            if (p == 1) __syncthreads();
-            for (; p + 1 < np; ++p) {
+        if (np > first) {
+            if (first) __syncthreads();
+            for (int p = first; p + 1 < np; ++p) {
                 // opaque per pass: otherwise every radix' loop-invariant
                 // address arithmetic is computed ahead of the loop (40
                 // instructions an element)

@@ -112,68 +112,68 @@ bool check_row(const Step& s, const Bufs& b, int64_t tw_count, std::string& why)
         if (!check_tile(a.ip, a.tfpc, 1, a.lpad, a.pshift, (int64_t)a.tfpc * a.lpad, a.nbuf, a.smem_bytes,
                         a.io_mode == IO_C2R_EVEN, a.io_mode == IO_R2C_EVEN, why)) return false;
     } else {
-    if (a.codelet < 0 && (a.ip.nthr * a.tfpc > maxthr || a.tfpc < 1)) return fail(why, "row threads");
-    if (a.tfpc < 1) return fail(why, "row tile");
-    if (a.nstage < 1 || a.nstage > 4) return fail(why, "row stages");
-    if (a.codelet >= 0) {
-        int cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
-        if (gfft_codelet_info(a.codelet, &cl, &cn, cr, &cnr, &cmaxt, &cminb) != 0 || cl != L || cn != a.ip.nthr ||
-            cnr != a.ip.npass)
-            return fail(why, "codelet mismatch");
-        for (int p = 0; p < cnr; ++p)
-            if (cr[p] != a.ip.pass[p].radix) return fail(why, "codelet radix mismatch");
-        if (a.nbuf != 1 && a.nbuf != 2) return fail(why, "codelet buffers");
-        bool need_tw = false;
-        for (int p = 0; p < a.ip.npass; ++p) need_tw |= a.ip.pass[p].ns > 1;
-        if (need_tw && a.tw_cnt == 0) return fail(why, "codelet twiddles not in shared memory");
-        const int ps = (cr[0] % 2 == 0) ? 4 : 30;
-        if (a.pshift != ps) return fail(why, "codelet padding");
-    }
+        if (a.codelet < 0 && (a.ip.nthr * a.tfpc > maxthr || a.tfpc < 1)) return fail(why, "row threads");
+        if (a.tfpc < 1) return fail(why, "row tile");
+        if (a.nstage < 1 || a.nstage > 4) return fail(why, "row stages");
+        if (a.codelet >= 0) {
+            int cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
+            if (gfft_codelet_info(a.codelet, &cl, &cn, cr, &cnr, &cmaxt, &cminb) != 0 || cl != L || cn != a.ip.nthr ||
+                cnr != a.ip.npass)
+                return fail(why, "codelet mismatch");
+            for (int p = 0; p < cnr; ++p)
+                if (cr[p] != a.ip.pass[p].radix) return fail(why, "codelet radix mismatch");
+            if (a.nbuf != 1 && a.nbuf != 2) return fail(why, "codelet buffers");
+            bool need_tw = false;
+            for (int p = 0; p < a.ip.npass; ++p) need_tw |= a.ip.pass[p].ns > 1;
+            if (need_tw && a.tw_cnt == 0) return fail(why, "codelet twiddles not in shared memory");
+            const int ps = (cr[0] % 2 == 0) ? 4 : 30;
+            if (a.pshift != ps) return fail(why, "codelet padding");
+        }
     }
     const bool even = a.io_mode == IO_R2C_EVEN || a.io_mode == IO_C2R_EVEN;
     const int maxidx = even ? L : L - 1;
     if (!a.tile) {
-    if (maxidx + (maxidx >> a.pshift) >= a.lpad) return fail(why, "row lpad too small");
-    const int64_t row_bytes = a.in_dist * a.in_esize;
-    if ((int64_t)a.tfpc * row_bytes > a.stage_bytes || a.stage_bytes % 16) return fail(why, "row stage too small");
-    if (a.codelet >= 0) {
-        int64_t slots_end = 64 + (int64_t)a.nstage * a.stage_bytes;
-        if (a.nbuf == 2) {  // work buffer after the slots, 16-byte aligned, lpad float2
-            if (a.smem_work < slots_end || a.smem_work % 16) return fail(why, "codelet work buffer");
-            slots_end = a.smem_work + (int64_t)a.lpad * 8;
+        if (maxidx + (maxidx >> a.pshift) >= a.lpad) return fail(why, "row lpad too small");
+        const int64_t row_bytes = a.in_dist * a.in_esize;
+        if ((int64_t)a.tfpc * row_bytes > a.stage_bytes || a.stage_bytes % 16) return fail(why, "row stage too small");
+        if (a.codelet >= 0) {
+            int64_t slots_end = 64 + (int64_t)a.nstage * a.stage_bytes;
+            if (a.nbuf == 2) {  // work buffer after the slots, 16-byte aligned, lpad float2
+                if (a.smem_work < slots_end || a.smem_work % 16) return fail(why, "codelet work buffer");
+                slots_end = a.smem_work + (int64_t)a.lpad * 8;
+            }
+            if (a.stage_bytes < a.in_dist * a.in_esize + 32 || a.stage_bytes < 16 + (int64_t)a.lpad * 8 || a.tfpc != 1)
+                return fail(why, "codelet slot too small");
+            int cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
+            gfft_codelet_info(a.codelet, &cl, &cn, cr, &cnr, &cmaxt, &cminb);
+            if (a.ngroups < 1 || a.ngroups > 15 || a.ngroups * a.ip.nthr > cmaxt) return fail(why, "codelet groups");
+            // tables arrive as 16-byte aligned supersets: one spare unit each
+            const int64_t tw_need = a.tw_cnt > 0 ? (int64_t)a.tw_cnt * 8 + 16 : 0;
+            const int64_t post_need = a.post_cnt > 0 ? (int64_t)a.post_cnt * 8 + 16 : 0;
+            if (a.smem_tw < 128 || a.smem_tw % 16 || a.smem_post % 16 || a.smem_post < a.smem_tw + tw_need ||
+                a.smem_stage < a.smem_post + post_need || a.smem_stage % 128 || a.group_bytes % 128 ||
+                a.stage_bytes % 16 || slots_end > a.group_bytes ||
+                a.smem_bytes < a.smem_stage + (int64_t)a.ngroups * a.group_bytes || a.smem_bytes > kMaxSmemBytes)
+                return fail(why, "codelet shared-memory layout");
+        } else if (a.smem_tw < 128 || a.smem_post < a.smem_tw + (int64_t)a.tw_cnt * 8 ||
+            a.smem_stage < a.smem_post + (int64_t)a.post_cnt * 8 || a.smem_stage % 16 ||
+            a.smem_work < a.smem_stage + (int64_t)a.nstage * a.stage_bytes ||
+            a.smem_bytes < a.smem_work + (int64_t)a.tfpc * a.nbuf * a.lpad * 8 || a.smem_bytes > kMaxSmemBytes)
+            return fail(why, "row shared-memory layout");
+        if (a.tw_cnt > 0) {
+            for (int p = 0; p < a.ip.npass; ++p) {
+                const PassDesc& d = a.ip.pass[p];
+                if (d.ns > 1 && (d.tw_off < a.tw_lo || d.tw_off + (int64_t)d.ns * d.radix > a.tw_lo + a.tw_cnt))
+                    return fail(why, "pass table outside the shared window");
+            }
+            if (a.tw_lo + (int64_t)a.tw_cnt > tw_count || a.tw_lo % 2) return fail(why, "twiddle window");
         }
-        if (a.stage_bytes < a.in_dist * a.in_esize + 32 || a.stage_bytes < 16 + (int64_t)a.lpad * 8 || a.tfpc != 1)
-            return fail(why, "codelet slot too small");
-        int cl = 0, cn = 0, cr[kMaxPass], cnr = 0, cmaxt = 0, cminb = 0;
-        gfft_codelet_info(a.codelet, &cl, &cn, cr, &cnr, &cmaxt, &cminb);
-        if (a.ngroups < 1 || a.ngroups > 15 || a.ngroups * a.ip.nthr > cmaxt) return fail(why, "codelet groups");
-        // tables arrive as 16-byte aligned supersets: one spare unit each
-        const int64_t tw_need = a.tw_cnt > 0 ? (int64_t)a.tw_cnt * 8 + 16 : 0;
-        const int64_t post_need = a.post_cnt > 0 ? (int64_t)a.post_cnt * 8 + 16 : 0;
-        if (a.smem_tw < 128 || a.smem_tw % 16 || a.smem_post % 16 || a.smem_post < a.smem_tw + tw_need ||
-            a.smem_stage < a.smem_post + post_need || a.smem_stage % 128 || a.group_bytes % 128 ||
-            a.stage_bytes % 16 || slots_end > a.group_bytes ||
-            a.smem_bytes < a.smem_stage + (int64_t)a.ngroups * a.group_bytes || a.smem_bytes > kMaxSmemBytes)
-            return fail(why, "codelet shared-memory layout");
-    } else if (a.smem_tw < 128 || a.smem_post < a.smem_tw + (int64_t)a.tw_cnt * 8 ||
-        a.smem_stage < a.smem_post + (int64_t)a.post_cnt * 8 || a.smem_stage % 16 ||
-        a.smem_work < a.smem_stage + (int64_t)a.nstage * a.stage_bytes ||
-        a.smem_bytes < a.smem_work + (int64_t)a.tfpc * a.nbuf * a.lpad * 8 || a.smem_bytes > kMaxSmemBytes)
-        return fail(why, "row shared-memory layout");
-    if (a.tw_cnt > 0) {
-        for (int p = 0; p < a.ip.npass; ++p) {
-            const PassDesc& d = a.ip.pass[p];
-            if (d.ns > 1 && (d.tw_off < a.tw_lo || d.tw_off + (int64_t)d.ns * d.radix > a.tw_lo + a.tw_cnt))
-                return fail(why, "pass table outside the shared window");
+        if (a.codelet < 0) {
+            const int start = a.io_mode == IO_C2R_EVEN ? 1 : 0;
+            const bool last_global = !(a.io_mode == IO_R2C_EVEN || (a.io_mode == IO_C2C && a.staged));
+            if (buffers_used(a.ip.npass, start, last_global) > a.nbuf) return fail(why, "row needs more shared buffers");
         }
-        if (a.tw_lo + (int64_t)a.tw_cnt > tw_count || a.tw_lo % 2) return fail(why, "twiddle window");
-    }
-    if (a.codelet < 0) {
-        const int start = a.io_mode == IO_C2R_EVEN ? 1 : 0;
-        const bool last_global = !(a.io_mode == IO_R2C_EVEN || (a.io_mode == IO_C2C && a.staged));
-        if (buffers_used(a.ip.npass, start, last_global) > a.nbuf) return fail(why, "row needs more shared buffers");
-    }
-    if (a.staged && (int64_t)a.tfpc * (L + 1) >= (1 << 22)) return fail(why, "staged copy index range");
+        if (a.staged && (int64_t)a.tfpc * (L + 1) >= (1 << 22)) return fail(why, "staged copy index range");
     }
     int64_t in_last = 0, out_last = 0, in_es = 8, out_es = 8;
     const int N = a.nreal;
