@@ -3,15 +3,17 @@
 // scheme of tile_fft.cuh on double2), with the even/odd post-process of a D2Z
 // and the Hermitian pre-process of a Z2D on chip.
 //
-// What bounds it: GB300's FP64 pipe, a small fraction of its FP32 rate.  The
-// one-launch-per-radix passes of dfft.cu kept that pipe 78 % busy and wrote
-// every intermediate to HBM.  Here a warp instruction's lanes are what counts:
+// What bounds it: GB300's FP64 pipe, a small fraction of its FP32 rate: 82 %
+// busy (D2Z 3000 x 2048).  The one-launch-per-radix passes of dfft.cu kept it 78 %
+// busy and wrote every intermediate to HBM.  Here a warp instruction's lanes are what counts:
 // butterflies of several rows share warps (1000 points, 100 butterflies a
 // pass: 3.2 warps' worth instead of 4).  Measured, one launch per radix ->
 // this: Z2Z 4096 x 2048 912 -> 689 us, 1000 x 4096 415 -> 362 (398 with a row
 // to every warp group), 300 x 1280 42 -> 33, D2Z 3000 x 2048 394 -> 320, Z2D
 // 372 -> 333, Z2Z 1500 x 64 51 -> 27.  Registers and residency make no
-// difference (80, 64 or 128 registers: 688, 691, 700 us).
+// difference (80, 64 or 128 registers: 688, 691, 700 us), although 80 spill
+// (272 bytes of stack, 2.3 KB of loads over all radices).  Columns: 2D Z2Z 1024^2
+// 228 -> 165, 500 x 16 x 64 60 -> 48 (32 columns; 93 with 8).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

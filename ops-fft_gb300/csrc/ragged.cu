@@ -27,9 +27,11 @@
 //
 // What bounds it: issue and latency at 32 warps per SM (issue 30 % active,
 // warps waiting on loads 5.9, at barriers 4.6 per issue).  10000 transforms
-// of 16..32768 points: 977 -> 419 us against the staged shared-memory passes
-// this replaced; 163 of up to 8192, one or two items a CTA with cold code,
-// 17.2 -> 19.9.  Measured and left out: CTAs of 256 threads, four per SM
+// of 16..32768 points: 977 -> 415 us against the staged shared-memory passes
+// this replaced; 163 of up to 8192, one item a CTA with cold code, 17.0 -> 18.8.
+// 64 registers spill (128 bytes of stack, 2.9 KB of loads over all radices).
+// Measured and left out: the passes specialised by item kind, with a tenth of
+// the spills, 163 transforms 26.7 us, 10000 653 (three copies of them); CTAs of 256 threads, four per SM
 // (one length 10 % faster, mixed lengths 516 us); HBM reads started one round
 // of the grid ahead with bulk L2 prefetches (515 us); one copy of each radix'
 // code for first, inner and last passes (559 us).

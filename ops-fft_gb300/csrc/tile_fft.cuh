@@ -25,7 +25,8 @@
 // element, whatever the length.
 //
 // What bounds it: latency, hidden by resident threads.  64 registers a
-// thread (no spills) keep 1024 threads per SM, 128 KB of loads when all of
+// thread (no spills but in the odd real modes: 540 bytes of loads R2C, 368 C2R)
+// keep 1024 threads per SM, 128 KB of loads when all of
 // them load, in CTAs small enough that one's loads overlap another's passes.
 // Measured (GB300, share of the measured copy bandwidth, 128 -> 64
 // registers): 256 x 263168 columns 232 -> 168 us (0.945), 2310 x 4096 rows

@@ -497,7 +497,8 @@ bool codelet_asked(int io_mode)
 // 4096 44 / 55; R2C 1024 x 64 2.4 / 3.5, 3000 x 64 3.2 / 3.9, 3000 x 4096 23.3
 // / 27.7, 8192 x 4096 54 / 86; C2R 1024 x 64 2.7 / 3.4, 3000 x 4096 27.6 /
 // 28.0, 8192 x 4096 61 / 88.  The codelets keep pinned host buffers used in
-// place, tuned plans and 8192 points (C2R 16384: clusters below 1024 rows).
+// place, chunked host calls, plans tuned to one of them (a tuned plan may also
+// stay here) and 8192 points (C2R 16384: clusters below 1024 rows).
 bool tile_beats_codelet(int L, int io_mode) { return L <= 4096 && !codelet_asked(io_mode); }
 
 // Rows of any length with radices <= 16 on the tile kernel.
@@ -1785,8 +1786,8 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         // two passes over HBM beat a 16-CTA cluster from 8 rows (us, 131072:
         // R2C x 1 8.9 / 8.6, x 8 10.4 / 11.7, x 64 33 / 46, x 512 223 / 316;
         // C2R x 512 242 / 323); 65536: R2C 114 / 118, C2R 125 / 123.  Out of
-        // place the middle result sits in the output, in place in the
-        // workspace that the cluster's copy needs too.
+        // place the middle result sits in the output, in place in the workspace
+        // (which the plan holds for both) that the cluster's copy needs too.
         if (L == 65536 && p.batch >= 8 && row_tile_beats_cluster(mode)) {
             const std::vector<int> fac = split_axis(L, cap);
             if (fac.size() == 2 && make_pair_steps(L, p.batch, r2c, p.weight, IN, inplace ? BUF_WS : BUF_OUT,
@@ -1819,8 +1820,8 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
             }
         }
         if (row_ok) return single(mode, (int)L, r2c ? L : nb, r2c ? nb : L);
-        // long real transforms: two passes with the packing on chip; out of
-        // place the middle result sits in the output rows
+        // long real transforms: two passes with the packing on chip, the middle
+        // result in a workspace
         {
             const std::vector<int> fac = split_axis(L, cap);
             if (fac.size() == 2 &&
