@@ -228,6 +228,7 @@ namespace {
 // (csrc/tile_fft.cuh)
 constexpr int kTileMaxThreads = 512;
 constexpr int kTileElems = 16;  // elements a thread holds
+constexpr int kSMs = 152;       // of a GB300: the rules for small batches count CTAs and threads per SM
 constexpr int64_t kTileMaxCols = (int64_t(1) << 31) - 64;  // 32-bit column arithmetic
 
 }  // namespace
@@ -520,7 +521,7 @@ bool make_tile_row_step(int L, int64_t ntf, int64_t in_dist, int64_t out_dist, i
     // at most 256 threads on an SM
     int T1 = 1;
     for (int r : rad) T1 = std::max(T1, L / r);
-    if (T1 <= kTileMaxThreads && ntf * T1 <= 152 * 256) T = T1;
+    if (T1 <= kTileMaxThreads && ntf * T1 <= kSMs * 256) T = T1;
     TwiddleBuilder trial = tb;
     st = Step{};
     st.kind = Step::ROW;
@@ -717,13 +718,13 @@ bool make_tile_col(int64_t S, int Lq, int64_t Ns, bool staged_out, TwiddleBuilde
     // 2D R2C 25 x 128 x 30 8.0 / 5.4, C2R 10 x 256 x 256 12.2 / 8.2, 1 x 512 x 256
     // 11.3 / 7.6, C2C 22 x 512 x 100 13.8 / 11.4)
     auto compiled = [&](int w) { return tile_compiled(false, Lq, T, w, rad); };
-    while (W > 4 && a.ncols / W < 304 && (!compiled(W) || compiled(W / 2))) W >>= 1;
+    while (W > 4 && a.ncols / W < 2 * kSMs && (!compiled(W) || compiled(W / 2))) W >>= 1;
     // and, as for rows, a thread for every butterfly while that leaves at most
     // 256 threads on an SM (us, without / with: 32 x 30 2D 7.1 / 5.3, 32 x 30 x
     // 40 12.3 / 9.9)
     int T1 = 1;
     for (int r : rad) T1 = std::max(T1, Lq / r);
-    if (!compiled(W) && T1 * W <= kTileMaxThreads && a.ncols * T1 <= 152 * 256) T = T1;
+    if (!compiled(W) && T1 * W <= kTileMaxThreads && a.ncols * T1 <= kSMs * 256) T = T1;
     TwiddleBuilder trial = tb;
     InnerPlan ip;
     if (!build_inner(Lq, rad, T, trial, ip)) return false;
@@ -806,10 +807,10 @@ bool make_pair_steps(int64_t L, int64_t batch, bool r2c, int weight, int src, in
     // for every butterfly (R2C, us: 30000 x 4 11.7 -> 10.4, 36000 x 1 11.9 -> 10.2)
     const int64_t pairs = batch * (L / Lq / 2 + 1);
     if (!pair_compiled(r2c, Lq, T, W, rad)) {
-        while (W > 8 && pairs / (W / 2) < 304) W >>= 1;
+        while (W > 8 && pairs / (W / 2) < 2 * kSMs) W >>= 1;
         int T1 = 1;
         for (int r : rad) T1 = std::max(T1, Lq / r);
-        if (T1 * W <= kTileMaxThreads && 2 * pairs * T1 <= 152 * 256) T = T1;
+        if (T1 * W <= kTileMaxThreads && 2 * pairs * T1 <= kSMs * 256) T = T1;
     }
     if (!build_inner(Lq, rad, T, trial, c.ip)) return false;
     c.pshift = tile_pshift(Lq, rad, !r2c);
@@ -1208,7 +1209,7 @@ bool make_dtile(int64_t n, int64_t ntf, bool t_fast, bool c2r, DPassArgs& a)
         while (W > 1 && W * T > kDTileThreads) W >>= 1;
         double best = cost(W, need);
         threads = (int)need;
-        for (int w = 2 * W; W >= 8 && w <= 32 && ntf / w >= 304 && w * lp * 16 <= 72 * 1024; w *= 2) {
+        for (int w = 2 * W; W >= 8 && w <= 32 && ntf / w >= 2 * kSMs && w * lp * 16 <= 72 * 1024; w *= 2) {
             const double c = cost(w, need);
             if (need > kDTileThreads) break;
             if (c < 0.95 * best) {
@@ -1229,7 +1230,7 @@ bool make_dtile(int64_t n, int64_t ntf, bool t_fast, bool c2r, DPassArgs& a)
                 W = w;
                 threads = (int)need;
             }
-            if (ntf / w < 304) break;
+            if (ntf / w < 2 * kSMs) break;
         }
         if (threads == 0) return false;
     }

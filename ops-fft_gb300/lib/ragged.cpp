@@ -47,7 +47,7 @@ constexpr int kMaxSingle = 4096;         // longest on-chip complex length
 constexpr int64_t kMaxLength = 1 << 24;
 constexpr int kOuterTable = 1 << 16;     // longest length with a whole outer-twiddle table (512 KB)
 constexpr int kPostPairs = 4096;         // bin pairs of one post-process item
-constexpr int kResident = 304;           // CTAs at once: two on each of 152 SMs
+constexpr int kResident = 2 * 152;       // CTAs at once: two on each SM of a GB300
 // workspace of one group of long transforms: the next group's first steps
 // are queued between a group's first and second steps, so the workspace in
 // flight is two groups and stays in the L2
