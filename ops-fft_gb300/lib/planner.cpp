@@ -1558,12 +1558,13 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         // strided axes of few points stay on the column kernel: a tile's code is
         // cold after that kernel's, and the passes are too short to make up for
         // it.  All axes or none (kernels of three kinds are colder still), none
-        // where a compiled tile waits, and of 2D transforms those of 17 to 90
-        // points (us, tiles / column kernel: 3D 60 x 21 x 19 19.0 / 16.1, 32 x 30 x
-        // 41 24.9 / 22.2, 21 x 125 x 41 27.7 / 25.6, 200 x 60 x 41 30.5 / 28.2, but
-        // 16 x 96 x 38 21.0 / 22.8; 2D 470 x 20 x 41 23.3 / 21.7, 2 x 80 x 86 20.3 /
-        // 18.9, but 1 x 75 x 34 15.4 / 16.1, 1 x 16 x 205 20.1 / 21.3, 1 x 300 x 86
-        // 25.5 / 26.3)
+        // where a compiled tile or an axis of 16 points, one pass without an
+        // exchange, waits, and of 2D transforms those of 17 to 90 points (us,
+        // tiles / column kernel: 3D 60 x 21 x 19 19.0 / 16.1, 32 x 30 x 41 24.9 /
+        // 22.2, 21 x 125 x 41 27.7 / 25.6, 200 x 60 x 41 30.5 / 28.2, 8 x 21 x 38 17.1
+        // / 15.1, but 16 x 96 x 38 20.9 / 22.8, 135 x 16 x 38 18.0 / 20.1; 2D 470 x
+        // 20 x 41 23.3 / 21.7, 2 x 80 x 86 20.3 / 18.9, but 1 x 75 x 34 15.4 / 16.1,
+        // 1 x 16 x 205 20.1 / 21.3, 1 x 300 x 86 25.5 / 26.3)
         const int64_t row_len = p.kind == Kind::C2C || last % 2 ? last : last / 2;
         const std::vector<int> row_rad = row_len <= row_max_length() ? choose_radices((int)row_len) : std::vector<int>{};
         bool column_kernel = !row_rad.empty() && *std::max_element(row_rad.begin(), row_rad.end()) > 16 &&
@@ -1572,7 +1573,7 @@ bool build_steps(const Problem& p, bool inplace, TwiddleBuilder& tb, StepList& o
         for (int a = 0; a + 1 < nd; ++a) strided += dims[a] > 1;
         for (int a = 0; a + 1 < nd && column_kernel; ++a) {
             const int64_t n = dims[a];
-            if (n > 1 && (n > cap || column_tile_compiled((int)n) || (strided == 1 && (n <= 16 || n > 90))))
+            if (n > 1 && (n > cap || n == 16 || column_tile_compiled((int)n) || (strided == 1 && (n < 16 || n > 90))))
                 column_kernel = false;
         }
 
