@@ -452,7 +452,7 @@ extern "C" int gfft_ragged_ctas(int smem_bytes)
     // the kernel's static shared memory counts against the opt-in limit, so
     // the attribute is a dynamic size actually launched with: the largest of
     // any plan on the device so far, since plans that asked for more are still
-    // launched
+    // launched (set each time: a device reset forgets it)
     static std::mutex mu;
     static int limit[64] = {0};
     int occ = 0, dev = 0;
@@ -460,10 +460,9 @@ extern "C" int gfft_ragged_ctas(int smem_bytes)
     if (e == cudaSuccess) {
         std::lock_guard<std::mutex> lk(mu);
         int& most = limit[dev & 63];
-        if (smem_bytes > most) {
-            e = cudaFuncSetAttribute(ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-            if (e == cudaSuccess) most = smem_bytes;
-        }
+        const int want = smem_bytes > most ? smem_bytes : most;
+        e = cudaFuncSetAttribute(ragged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+        if (e == cudaSuccess) most = want;
     }
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ragged_kernel, NT, (size_t)smem_bytes);
     if (e != cudaSuccess) {
